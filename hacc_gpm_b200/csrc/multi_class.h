@@ -67,7 +67,7 @@ struct MCTable {
 bool mc_class_supported(int ng, int np);
 
 cudaError_t mc_step(const MCTable& t, cudaStream_t s);
-// The FFT passes of mc_step (fft_passes.cu): z forward from the int64
+// The FFT passes of mc_step (fft_multi.cu): z forward from the int64
 // density, y forward, x with the Green's function, y inverse, z inverse to
 // the real potential.
 cudaError_t mc_launch_fft_passes(const MCTable& t, cudaStream_t s);

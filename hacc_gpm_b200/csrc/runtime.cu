@@ -1,7 +1,7 @@
 // runtime.cu — host runtime of the PM step behind the C-ABI (include/hgpm_c.h):
 // params parser, FP64 time stepper and growth factors, device memory of a
 // context, and the phase sequencing that launches the kernels of
-// particles.cu and fft_passes.cu on the context's stream.
+// particles.cu and the fft_*.cu passes on the context's stream.
 #include <cuda_runtime.h>
 
 #include <cmath>
