@@ -1819,17 +1819,44 @@ int kick_candidates(int np_side, int ng) {
 bool kick_uses_phi(int choice) { return choice >= kKickPhiFirst && choice < kKickCands; }
 bool kick_uses_phi2(int choice) { return choice == kKickPhi2; }
 
-// Measured mid-run, kick plus the z inverse phase that makes what it
-// gathers: 512^3 particles on 512^3 cells (16^3 blocks) 2.51 ms for the
-// paired potential, 2.73 for the real one, 2.78 for the force grid with its
-// gradient kernel; 512^3 on 1024^3 (8^3 blocks) 7.5 / 9.7 / 12.2 ms for the
-// real potential / the paired one / the force grid.
-int kick_default(int np_side, int ng) { return block_side(np_side, ng) == 16 ? kKickPhi2 : kKickPhiFirst; }
+// The paired potential for every shape.  Measured mid-run, kick plus the z
+// inverse phase that makes what it gathers: 512^3 particles on 512^3 cells
+// (16^3 blocks) 2.51 ms for the paired potential, 2.73 for the real one, 2.78
+// for the force grid with its gradient kernel; 8^3 blocks, paired against
+// real potential: 120^3 46 against 59 us, 200^3 168 against 220 us, 128^3 on
+// 256^3 104 against 110 us, 512^3 on 1024^3 5.84 against 6.3 ms (with the
+// short shares of kick_grid; with whole-kick shares it lost, 7.25 against
+// 6.64).
+int kick_default(int np_side, int ng) {
+    (void)np_side;
+    (void)ng;
+    return kKickPhi2;
+}
 
 int kick_kernels(int choice, int np_side, int ng) {
     (void)np_side;
     (void)ng;
     return choice == kKickWindowed ? 2 : 1;
+}
+
+// CTAs of a flat kick of `runs` runs, `resident` of them fitting the GPU at
+// once: whole waves of static shares, at least 9 runs each.  With one wave
+// (each CTA a resident's share of the whole kick) the kick is fastest alone,
+// but a CTA that finds its SM held by another stream starts when that lets
+// go and then has its whole share before it: of three contexts whose steps
+// overlap, kicks of 512^3 took 7-12 ms instead of 2.0.  Several waves leave
+// the balance to the block scheduler: 512^3 alone 2.00 / 2.04 / 2.05 / 2.06
+// ms a kick in 1 / 2 / 4 / 8 waves, four steps of three contexts in turn
+// 28.5 / 25.7 / 23.7 / 24.2 ms.  With more cells than particles a side
+// (8^3 blocks, CTAs of 256 threads whose turnover hides behind the other
+// three of the SM) short shares also keep the resident CTAs' gathers close
+// together: 512^3 particles on 1024^3 4.77 / 4.19 / 3.70 / 3.34 ms in 1 / 4 /
+// 8 / 55 waves.
+static int kick_grid(int runs, int resident, bool sparse) {
+    const int cap = sparse ? 64 : 4;
+    int waves = runs / resident / 9;
+    waves = waves < 1 ? 1 : waves > cap ? cap : waves;
+    return runs < resident * waves ? runs : resident * waves;
 }
 
 template <int B, int NT, int R>
@@ -1838,7 +1865,8 @@ static cudaError_t kick_flat_launch(const ParticleSoA& p, int np_side, int ng, c
                                     const KickSched& ks, int nslots, cudaStream_t s) {
     const int nblocks = (np_side / B) * (np_side / B) * (np_side / B);
     auto kf = kick_flat_nt_kernel<B, NT, R>;
-    const int grid = num_sms() * blocks_per_sm_once((const void*)kf, NT, 0);
+    const int resident = num_sms() * blocks_per_sm_once((const void*)kf, NT, 0);
+    const int grid = kick_grid(nblocks * (B * B * B / NT) / R, resident, ng > np_side);
     kf<<<dim3(grid, nslots), NT, 0, s>>>(p, ng, f, deltaT, fscal, pf_a, pf_b, ndrift, nblocks, sl, ks);
     return cudaGetLastError();
 }
@@ -1849,7 +1877,8 @@ static cudaError_t kick_phi_launch(const ParticleSoA& p, int np_side, int ng, co
                                    const KickSched& ks, int nslots, cudaStream_t s) {
     const int nblocks = (np_side / B) * (np_side / B) * (np_side / B);
     auto kf = kick_phi_kernel<B, NT, R, PAIR>;
-    const int grid = num_sms() * blocks_per_sm_once((const void*)kf, NT, 0);
+    const int resident = num_sms() * blocks_per_sm_once((const void*)kf, NT, 0);
+    const int grid = kick_grid(nblocks * (B * B * B / NT) / R, resident, ng > np_side);
     kf<<<dim3(grid, nslots), NT, 0, s>>>(p, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, nblocks, sl, ks);
     return cudaGetLastError();
 }
@@ -1860,14 +1889,26 @@ static cudaError_t kick_impl(const ParticleSoA& p, int np_side, int ng, const fl
                              bool have_rec, const SpillList& spill, const Slots& sl, const KickSched& ks, int nslots,
                              cudaStream_t s) {
     if (kick_uses_phi(choice)) {
+        // choice 6: runs of 2 units of the real potential, else runs of 4
+        // (16^3 blocks) or 1 (8^3 blocks)
         if constexpr (B == 16) {
+            // up to 96^3 (216 runs of four 1024-particle units for 148 SMs) a
+            // CTA takes 128 particles at a time, so that the box spreads over
+            // the GPU: 8.0 against 14.9 us at 32^3, 11.2 against 16.7 at 64^3,
+            // 22.3 against 24.1 at 96^3; at 128^3 40.7 against 39.3
+            if (np_side <= 96) {
+                if (choice == 7) return kick_phi_launch<B, 128, 1, true>(p, np_side, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, sl, ks, nslots, s);
+                return kick_phi_launch<B, 128, 1>(p, np_side, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, sl, ks, nslots, s);
+            }
             if (choice == 5) return kick_phi_launch<B, 1024, 4>(p, np_side, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, sl, ks, nslots, s);
             if (choice == 7) return kick_phi_launch<B, 1024, 4, true>(p, np_side, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, sl, ks, nslots, s);
             return kick_phi_launch<B, 1024, 2>(p, np_side, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, sl, ks, nslots, s);
         } else {
-            if (choice == 5) return kick_phi_launch<B, 512, 1>(p, np_side, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, sl, ks, nslots, s);
-            if (choice == 7) return kick_phi_launch<B, 512, 1, true>(p, np_side, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, sl, ks, nslots, s);
-            return kick_phi_launch<B, 512, 2>(p, np_side, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, sl, ks, nslots, s);
+            // 256 threads, half a block at a time: 33 us at 120^3, 133 at
+            // 200^3, as with 512, and shorter shares (kick_grid)
+            if (choice == 5) return kick_phi_launch<B, 256, 1>(p, np_side, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, sl, ks, nslots, s);
+            if (choice == 7) return kick_phi_launch<B, 256, 1, true>(p, np_side, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, sl, ks, nslots, s);
+            return kick_phi_launch<B, 256, 2>(p, np_side, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, sl, ks, nslots, s);
         }
     }
     constexpr int NT = 512;

@@ -359,3 +359,24 @@ def test_force_grid_on_demand_with_potential_kick(ng, np_side, monkeypatch):
     assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
     for st in states[1:]:
         assert np.array_equal(states[0][0], st[0]) and np.array_equal(states[0][1], st[1])
+
+
+@pytest.mark.parametrize("ng,np_side", [(96, 96), (120, 120), (256, 256), (256, 128), (320, 160)])
+def test_kick_shares_bit_identical(ng, np_side, monkeypatch):
+    """The potential-gathering kicks in 128-particle CTAs (up to 96^3), in
+    several waves of CTAs (256^3) and in 8^3 blocks give the flat force-grid
+    kick's state bit for bit."""
+    rng = np.random.default_rng(ng + np_side)
+    x = rng.random((np_side ** 3, 3), dtype=np.float32) * np.float32(ng * (1 - 2 ** -20))
+    v = rng.standard_normal((np_side ** 3, 3), dtype=np.float32)
+    out = []
+    for flag in ("3", "5", "6", "7"):
+        monkeypatch.setenv("HGPM_KICK", flag)
+        with make(ng, np_side) as s:
+            s.load_state(x, v)
+            s.cic()
+            s.solve_gradient()
+            s.kick_drift(0.0123, 1.7, 0.3, 0.25, 2)
+            out.append(s.store_state())
+    for o in out[1:]:
+        assert np.array_equal(out[0][0], o[0]) and np.array_equal(out[0][1], o[1])
