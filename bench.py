@@ -107,11 +107,11 @@ DEPOSIT_NAMES = {
          "deposit_w32_kernel<16,512,2,1>", "deposit_w32_kernel<16,256,4,1,4>", "deposit_col_kernel<16,4,4,0>",
          "deposit_col_kernel<16,4,2,0>", "deposit_col_kernel<16,3,4,0>",
          "deposit_col_kernel<16,4,4,1> (32-bit windows, x-half split, wraps from the atomics' returned values)",
-         "deposit_direct_kernel<16,S,512>", "deposit_col_kernel<16,4,4,2>",
+         "deposit_direct_kernel (a thread per particle, global atomics)", "deposit_col_kernel<16,4,4,2>",
          "deposit_col_kernel<16,4,4,1,1> (32-bit windows, x-half split, returned-value wraps, x-chain merge)"],
     8: ["deposit_tiled_kernel<8,S,256,3>", "deposit_w32_kernel<8,256,4,1,2> (32-bit windows, 13312 cells)",
         "deposit_col_kernel<8,12,4,0>", "deposit_w32_kernel<8,512,2,1,1>", "deposit_col_kernel<8,12,4,1>",
-        "deposit_direct_kernel<8,S,256>", "deposit_col_kernel<8,12,4,2>", "deposit_col_kernel<8,12,4,1,1>"],
+        "deposit_direct_kernel (a thread per particle, global atomics)", "deposit_col_kernel<8,12,4,2>", "deposit_col_kernel<8,12,4,1,1>"],
 }
 KICK_NAMES = {
     16: ["kick_flat_nt_kernel<16,1024,4> (float4 force gathers)", "kick_flat_nt_kernel<16,1024,2>",
@@ -121,8 +121,8 @@ KICK_NAMES = {
          "x-planes; 16 paired-potential gathers form the 8 corner forces)"],
     8: ["kick_spill_kernel<8>", "kick_flat_nt_kernel<8,512,1>", "kick_flat_nt_kernel<8,512,2>",
         "kick_flat_nt_kernel<8,256,4>", "kick_win4_kernel<8,512> + kick_spill_kernel<8>",
-        "kick_phi_kernel<8,512,1,0> (32 potential gathers form the 8 corner forces)", "kick_phi_kernel<8,512,2,0>",
-        "kick_phi_kernel<8,512,1,1> (paired potential)"],
+        "kick_phi_kernel<8,256,1,0> (32 potential gathers form the 8 corner forces)", "kick_phi_kernel<8,256,2,0>",
+        "kick_phi_kernel<8,256,1,1> (paired potential)"],
 }
 
 
@@ -139,7 +139,7 @@ def kernel_names(tuned, np_side, ng, plane=None):
         kick, "zpass_c2r_kernel<NG> (the potential) + gradient_kernel<8,3,2> (central differences, float4 force)")
     spill = "deposit_spill_kernel<%d,S,%d>" % (blk, 1024 if blk == 16 else 512)
     names = {
-        "deposit": "%s + %s (queued blocks)" % (DEPOSIT_NAMES[blk][dep], spill),
+        "deposit": DEPOSIT_NAMES[blk][dep] + ("" if dep == (9 if blk == 16 else 5) else " + %s (queued blocks)" % spill),
         "fft_z_fwd": "zpass_r2c_kernel<NG,1>",
         "fft_y_fwd": "strided_tma_kernel<NG,0,0>" if ypass else "strided_kernel<NG,0>",
         "poisson_x": {0: "xfused_kernel<NG,PotentialOp>", 1: "xpotential_tma_kernel<NG,256>"}.get(

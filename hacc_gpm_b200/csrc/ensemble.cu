@@ -430,9 +430,11 @@ extern "C" int hgpm_ens_release(hgpm_ensemble* E, int ci, int slot) {
     return HGPM_OK;
 }
 
-// Kernels of one class step besides the kick: deposit 2, z forward, y
-// forward, x potential, y inverse, z inverse, gradient, slot advance.
-constexpr int kStepKernels = 9;
+// Kernels of one class step: deposit (with its spill pass 2), z forward, y
+// forward, x potential, y inverse, z inverse, gradient, kick, slot advance.
+static int step_kernels(const hgpm_ensemble* E, const EnsClass& k) {
+    return 7 + (deposit_records(E->dep_choice, k.np, k.ng) ? 2 : 1) + kick_kernels(E->kick_choice, k.np, k.ng);
+}
 
 // All phases of one step for every slot of class k, on stream s.
 static int class_step(hgpm_ensemble* E, EnsClass& k, cudaStream_t s) {
@@ -464,11 +466,12 @@ static int class_step(hgpm_ensemble* E, EnsClass& k, cudaStream_t s) {
     ECK(launch_zinv(ng, k.fspec, phi, ng * ng, k.zs, 0, 0, 1, 1.0f, k.tw_ng, s,
                     Slots{act, 3 * k.spec_elems, 6 * k.spec_elems}, S));
     ECK(launch_gradient(ng, phi, f4, s, Slots{act, 6 * k.spec_elems, k.force_elems / 4}, S));
-    ECK(launch_kick_drift(p, k.np, ng, f4, 0.0, 0.0, 0.f, 0.f, 0, E->kick_choice, k.blkwin, true, k.kick_spill, s,
+    ECK(launch_kick_drift(p, k.np, ng, f4, 0.0, 0.0, 0.f, 0.f, 0, E->kick_choice, k.blkwin,
+                          deposit_records(E->dep_choice, k.np, ng), k.kick_spill, s,
                           Slots{act, k.part_stride, k.force_elems / 4, k.win_stride},
                           KickSched{k.d_sched, k.d_step, HGPM_MAX_STEPS}, S));
     ECK(launch_slots_advance(k.d_active, k.d_step, k.d_nsteps, S, s));
-    E->launches += kStepKernels + kick_kernels(E->kick_choice, k.np, ng);
+    E->launches += step_kernels(E, k);
     return HGPM_OK;
 }
 
@@ -603,7 +606,7 @@ extern "C" int hgpm_ens_step(hgpm_ensemble* E, int nsteps) {
         int per = 0;
         if (multi_ok(E)) per = kMCStepLaunches;
         else
-            for (auto& k : E->cls) per += kStepKernels + kick_kernels(E->kick_choice, k.np, k.ng);
+            for (auto& k : E->cls) per += step_kernels(E, k);
         for (int i = 0; i < nsteps; ++i) {
             ECK(cudaGraphLaunch(E->exec, E->stream));
             E->launches += per;
@@ -654,7 +657,7 @@ extern "C" int hgpm_ens_step_class(hgpm_ensemble* E, int ci, int nsteps) {
         }
         for (int i = 0; i < nsteps; ++i) {
             ECK(cudaGraphLaunch(k.exec, k.stream));
-            E->launches += kStepKernels + kick_kernels(E->kick_choice, k.np, k.ng);
+            E->launches += step_kernels(E, k);
         }
     } else {
         for (int i = 0; i < nsteps; ++i)

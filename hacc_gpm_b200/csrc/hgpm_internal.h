@@ -125,6 +125,9 @@ bool kick_uses_phi2(int choice);
 // default (used when the choice is -1).
 int deposit_candidates(int np_side, int ng);
 int deposit_default(int np_side, int ng);
+// Whether candidate `choice` writes the blocks' window records and launches a
+// spill pass (all but the direct one).
+bool deposit_records(int choice, int np_side, int ng);
 // Built-in kick candidate (without tuning): the paired potential for 16^3
 // blocks, the real potential for 8^3 blocks.
 int kick_default(int np_side, int ng);

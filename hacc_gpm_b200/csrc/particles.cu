@@ -808,40 +808,21 @@ __device__ __forceinline__ void deposit_global(unsigned long long* __restrict__ 
             for (int cc = 0; cc < 2; ++cc) atomicAdd(&rho[sx[a] + sy[b] + sz[cc]], q[(a * 2 + b) * 2 + cc]);
 }
 
-// Direct deposit: one CTA per Lagrangian block records the block's window
-// (for the windowed kick, as the windowed deposits do), then every particle
-// adds its 8 fixed-point weights straight to the int64 grid.  Where a window
-// would hold about one contribution per cell (more cells than particles per
-// axis: each particle's corners are mostly its own) this skips the window's
-// zeroing and flush; the sums are the same integers (bit-identical grids).
-template <int B, bool SMALL, int NT>
-__global__ void __launch_bounds__(NT) deposit_direct_kernel(ParticleSoA p, int np_side, int ng, float mass,
-                                                            unsigned long long* __restrict__ rho, int cap_cells,
-                                                            int* __restrict__ blkwin, SpillList spill, Slots sl) {
-    constexpr int B3 = B * B * B;
-    constexpr int PPT = B3 / NT;
-    static_assert(B3 % NT == 0, "whole particles per thread");
-    (void)cap_cells;
-    __shared__ int bb[6];
+// Direct deposit: a thread per particle adds its 8 fixed-point weights
+// straight to the int64 grid; no window, no window records, no spill pass and
+// no counters to clear.  The sums are the same integers (bit-identical grids).
+// Bound by the L2's atomics (about 480 G/s), so it loses to the windows once
+// these have a block for every SM, and wins where they do not (see
+// deposit_default_choice).
+template <bool SMALL>
+__global__ void __launch_bounds__(128) deposit_direct_kernel(ParticleSoA p, int n, int ng, float mass,
+                                                             unsigned long long* __restrict__ rho, Slots sl) {
     if (slot_idle(sl, blockIdx.y)) return;
-    const int tid = threadIdx.x;
-    const int nb = np_side / B;
-    const int blk = blockIdx.x;
-    p = offset_soa(p, (size_t)blockIdx.y * sl.s0 + (size_t)blk * B3);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    p = offset_soa(p, (size_t)blockIdx.y * sl.s0);
     rho += (size_t)blockIdx.y * sl.s1;
-    const int bz = blk % nb, by = (blk / nb) % nb, bx = blk / (nb * nb);
-    const int ox = (int)((long long)bx * B * ng / np_side);
-    const int oy = (int)((long long)by * B * ng / np_side);
-    const int oz = (int)((long long)bz * B * ng / np_side);
-    int l0[3], w[3];
-    block_window<NT, PPT>(p.cell, 0, ox, oy, oz, ng, bb, l0, w);
-    if (blkwin && tid < 6) blkwin[(size_t)blockIdx.y * sl.s2 + (size_t)blk * kWinRec + tid] = tid < 3 ? l0[tid] : w[tid - 3];
-    if (tid == 0 && spill.over && (long long)w[0] * w[1] * w[2] > kWin4Cap) atomicAdd(&spill.over[blockIdx.y], 1);
-#pragma unroll 2
-    for (int k = 0; k < PPT; ++k) {
-        const int i = tid + k * NT;
-        deposit_global<SMALL>(rho, __ldg(&p.cell[i]), __ldg(&p.ox[i]), __ldg(&p.oy[i]), __ldg(&p.oz[i]), mass, ng);
-    }
+    deposit_global<SMALL>(rho, __ldg(&p.cell[i]), __ldg(&p.ox[i]), __ldg(&p.oy[i]), __ldg(&p.oz[i]), mass, ng);
 }
 
 // Blocks queued by deposit_tiled_kernel (window wider than its own): a
@@ -1664,7 +1645,7 @@ static int num_sms() {
 
 // Windowed deposit configurations.  The kernels share one signature; a
 // configuration is (kernel, threads per CTA, window cells, bytes per window
-// cell).
+// cell); no kernel: deposit_direct_kernel.
 using DepositFn = void (*)(ParticleSoA, int, int, float, unsigned long long*, int, int*, SpillList, Slots);
 struct DepositCfg {
     DepositFn fn;
@@ -1710,7 +1691,7 @@ static int deposit_candidates(int cap_default, bool w32, DepositCfg* out) {
             for (int i = 0; i < 6; ++i) out[n + i] = out[same_nt[i]];
             n += 6;
         }
-        out[n++] = {deposit_direct_kernel<B, SMALL, 512>, 512, 0, 0};
+        out[n++] = {nullptr, 0, 0, 0};
         out[n++] = w32 ? DepositCfg{deposit_col_kernel<B, 4, 4, 2>, 256, 13312, 4} : out[0];
         out[n++] = w32 ? DepositCfg{deposit_col_kernel<B, 4, 4, 1, true>, 256, 13312, 4} : out[0];
     } else {
@@ -1723,24 +1704,31 @@ static int deposit_candidates(int cap_default, bool w32, DepositCfg* out) {
         } else {
             for (int i = 0; i < 4; ++i) out[n++] = out[0];
         }
-        out[n++] = {deposit_direct_kernel<B, SMALL, 256>, 256, 0, 0};
+        out[n++] = {nullptr, 0, 0, 0};
         out[n++] = w32 ? DepositCfg{deposit_col_kernel<B, 12, 4, 2>, B * B, 4096, 4} : out[0];
         out[n++] = w32 ? DepositCfg{deposit_col_kernel<B, 12, 4, 1, true>, B * B, 4096, 4} : out[0];
     }
     return n;
 }
 
-// Default candidate (measured mid-run): 16^3 blocks the column kernel with
-// returned-value wrap detection (1.41 ms at 512^3, against 1.46 with the
-// window-sum check and 2.22 for the split window with 512 threads); 8^3
-// blocks with more cells than particles per axis (their windows span twice
-// the block) the 32-bit 256-thread kernel with 13312-cell windows (6.9 ms
-// for 512^3 particles on a 1024^3 grid, against 8.3-11.8 for the other
-// windows), otherwise the column kernel.
+// Default candidate (measured mid-run).  Small boxes, whose blocks are too few
+// for the GPU's SMs: the direct deposit.  us a deposit with its spill pass and
+// counters, windowed / direct, 16^3 blocks: 40 / 8 at 32^3, 37 / 16 at 64^3,
+// 36 / 27 at 96^3, 40 / 53 at 128^3; 8^3 blocks: 21 / 9 at 40^3, 35 / 45 at
+// 120^3; 8^3 blocks and twice the particles' side of cells: 27 / 7 for 32^3,
+// 36 / 17 for 64^3, 109 / 91 for 128^3, 5002 / 6099 for 512^3.  Else, 16^3
+// blocks: the column kernel with returned-value wrap detection (1.41 ms at
+// 512^3, against 1.46 with the window-sum check and 2.22 for the split window
+// with 512 threads); 8^3 blocks with more cells than particles per axis (their
+// windows span twice the block) the 32-bit 256-thread kernel with 13312-cell
+// windows (6.9 ms for 512^3 particles on a 1024^3 grid, against 8.3-11.8 for
+// the other windows), otherwise the column kernel (returned-value wraps 103.6
+// us at 200^3, window-sum check 106.7).
 template <int B>
 static int deposit_default_choice(int np_side, int ng) {
-    if (B == 16) return 8;
-    return ng > np_side ? 1 : 2;
+    if (B == 16) return np_side <= 96 ? 9 : 8;
+    if (ng > np_side) return np_side <= 128 ? 5 : 1;
+    return np_side <= 64 ? 5 : 4;
 }
 
 template <int B, bool SMALL>
@@ -1752,6 +1740,11 @@ static cudaError_t deposit_impl(const ParticleSoA& p, int np_side, int ng, float
     const int mode = choice >= 0 && choice < ncand ? choice : deposit_default_choice<B>(np_side, ng);
     const DepositCfg& cfg = cands[mode];
     const DepositFn k = cfg.fn;
+    if (!k) {  // direct: n <= 1024^3
+        const int n = np_side * np_side * np_side;
+        deposit_direct_kernel<SMALL><<<dim3(nblk(n, 128), nslots), 128, 0, s>>>(p, n, ng, mass, rho, sl);
+        return cudaGetLastError();
+    }
     const int nt = cfg.nt;
     cap = cfg.cap;
     const int smem = cap * cfg.cell_bytes;
@@ -1771,6 +1764,11 @@ static cudaError_t deposit_impl(const ParticleSoA& p, int np_side, int ng, float
     const int per_slot = num_sms() / nslots > 1 ? num_sms() / nslots : 1;  // about one CTA per SM in all
     ks<<<dim3(per_slot, nslots), NTS, kBigCap * 8, s>>>(p, np_side, ng, mass, rho, blkwin, spill, sl);
     return cudaGetLastError();
+}
+
+bool deposit_records(int choice, int np_side, int ng) {
+    if (choice < 0 || choice >= deposit_candidates(np_side, ng)) choice = deposit_default(np_side, ng);
+    return choice != (block_side(np_side, ng) == 16 ? 9 : 5);
 }
 
 int deposit_candidates(int np_side, int ng) { return block_side(np_side, ng) == 16 ? kDepositCands : 8; }

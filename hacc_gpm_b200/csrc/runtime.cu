@@ -705,8 +705,8 @@ static int deposit_impl(hgpm_ctx* c) {
     if (c->rho_dirty) CK(cudaMemsetAsync(c->rho64, 0, c->ncell * 8, c->stream));
     CK(launch_deposit(c->part, c->np, c->ng, cic_mass(c->ng, c->np), c->rho64, c->blkwin, c->dep_spill, c->stream,
                       Slots{}, 1, c->dep_choice));
-    c->win_valid = true;
-    count(c, PH_DEPOSIT, 2);  // windowed pass + spill pass
+    c->win_valid = deposit_records(c->dep_choice, c->np, c->ng);
+    count(c, PH_DEPOSIT, c->win_valid ? 2 : 1);  // windowed pass + spill pass, or the direct one
     c->rho_dirty = true;
     return HGPM_OK;
 }

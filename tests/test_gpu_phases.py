@@ -380,3 +380,23 @@ def test_kick_shares_bit_identical(ng, np_side, monkeypatch):
             out.append(s.store_state())
     for o in out[1:]:
         assert np.array_equal(out[0][0], o[0]) and np.array_equal(out[0][1], o[1])
+
+
+@pytest.mark.parametrize("ng,np_side", [(96, 96), (128, 128), (40, 40), (120, 120), (256, 128), (320, 160)])
+def test_default_deposit_on_each_side_of_its_rule(ng, np_side, monkeypatch):
+    """The default deposit (direct below its rule's sides, windowed above)
+    gives the split window's grid bit for bit, twice in a row."""
+    x, v = lattice_state(np_side, ng, disp=2.5, vel=1.0, seed=41)
+    out = []
+    for flag in ("0", None):
+        if flag is None:
+            monkeypatch.delenv("HGPM_DEPOSIT", raising=False)
+        else:
+            monkeypatch.setenv("HGPM_DEPOSIT", flag)
+        with make(ng, np_side) as s:
+            s.load_state(x, v)
+            for _ in range(2):
+                s.cic()
+                out.append(s.get_density())
+    for o in out[1:]:
+        assert np.array_equal(out[0], o)
