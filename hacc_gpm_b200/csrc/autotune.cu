@@ -12,7 +12,7 @@
 //            is charged to the others), CTA shape, units per CTA turn
 //            (launch_kick_drift candidates),
 //   y pass   TMA-fed persistent or plain strided transform,
-//   x pass   TMA-fed persistent or plain fused Poisson transform.
+//   x pass   TMA-fed persistent or line-tile fused Poisson transform.
 // hgpm_autotune times every candidate on the context's own current state
 // (CUDA events on its stream), keeps the default unless another candidate
 // is faster by more than the noise margin, applies the winners to the
@@ -221,8 +221,7 @@ extern "C" int hgpm_autotune(hgpm_ctx* c, int reps, int store, int choices[HGPM_
         pick[HGPM_TUNE_YPASS] = hgpm_tune_pick(ms, 2, 1, tol);
         pms[HGPM_TUNE_YPASS] = ms[pick[HGPM_TUNE_YPASS]];
     }
-    // x pass with the Green's function: 0 = plain, 1 = TMA-fed, 2 = plain
-    // with twice the columns per CTA
+    // x pass with the Green's function: 1 = TMA-fed, 0 and 2 = the line tiles
     {
         double ms[3];
         const double coeff = 0.5 / ((double)ng * ng * ng);
@@ -231,11 +230,7 @@ extern "C" int hgpm_autotune(hgpm_ctx* c, int reps, int store, int choices[HGPM_
                 if (t == 1)
                     return launch_xpotential_tma(ng, c->spec, c->fspec, M + 1, c->zs, c->tw_ng, c->cosq, coeff,
                                                  c->d_err + 1, c->stream);
-                if (t == 2)
-                    return launch_xpotential_wide(ng, c->spec, c->fspec, M + 1, (size_t)ng * c->zs, (size_t)c->zs,
-                                                  ng, c->tw_ng, c->cosq, coeff, c->stream);
-                return launch_xpotential(ng, c->spec, c->fspec, M + 1, (size_t)ng * c->zs, (size_t)c->zs, ng,
-                                         c->tw_ng, c->cosq, coeff, c->stream);
+                return launch_xpotential(ng, c->spec, c->fspec, c->zs, c->tw_ng, c->cosq, coeff, c->stream);
             }, &e);
             CK(e);
         }

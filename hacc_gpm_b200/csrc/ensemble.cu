@@ -457,8 +457,8 @@ static int class_step(hgpm_ensemble* E, EnsClass& k, cudaStream_t s) {
     ECK(launch_zfwd(ng, k.rho64, true, k.spec, ng * ng, k.zs, mean, k.tw_ng, s, Slots{act, k.ncell, k.spec_elems}, S));
     ECK(launch_strided(ng, false, k.spec, M + 1, (size_t)k.zs, (size_t)ng * k.zs, ng, 0, 1, k.tw_ng, s,
                        Slots{act, k.spec_elems, 0}, S));
-    ECK(launch_xpotential(ng, k.spec, k.fspec, M + 1, (size_t)ng * k.zs, (size_t)k.zs, ng, k.tw_ng, k.cosq,
-                          0.5 / ((double)ng * ng * ng), s, Slots{act, k.spec_elems, 3 * k.spec_elems}, S));
+    ECK(launch_xpotential(ng, k.spec, k.fspec, k.zs, k.tw_ng, k.cosq, 0.5 / ((double)ng * ng * ng), s,
+                          Slots{act, k.spec_elems, 3 * k.spec_elems}, S));
     ECK(launch_strided(ng, true, k.fspec, M + 1, (size_t)k.zs, (size_t)ng * k.zs, ng, 0, 1, k.tw_ng, s,
                        Slots{act, 3 * k.spec_elems, 0}, S));
     float4* f4 = reinterpret_cast<float4*>(k.force);

@@ -314,4 +314,188 @@ __device__ __forceinline__ void fft_tile_fwd_op_inv(float2* buf, const float2* _
     fft_stages<N, C, ES, true, NT, TWS, TP, RL>(buf, tw, typename SeqRev<Init>::type{});
 }
 
+// ---- transforms in register groups ----------------------------------------
+// fft_tile stages the tile through shared memory once per radix and once more
+// on each side for the global loads and stores.  The group transforms below run
+// the same butterflies in the same order (bit for bit), but
+//   - consecutive radices whose product is at most kMaxGroup run in one
+//     thread's registers (a group, e.g. 1024 = 8, 8, 4x4),
+//   - the first group reads its elements where the data is (ld) and the last
+//     one leaves them where they go (st), so the tile crosses shared memory
+//     only between groups: 2 exchanges instead of 5 for 1024 points, and none
+//     for 16.
+// A group of radices R1, R2 (G = R1 R2) after stages of product NS owns
+// elements j + s N/G, s < G: the R2 butterflies j + r' N/G of the radix-R1
+// stage take s = r' + r R2, and their outputs r are the inputs of R1
+// butterflies of the radix-R2 stage.  Its outputs q land at
+// (j / NS) NS G + j % NS + q NS, as a radix-G Stockham stage's.
+constexpr int kMaxGroup = 16;
+
+template <class... Gs> struct GList {};
+template <class S> struct SeqProd;
+template <> struct SeqProd<RSeq<>> { static constexpr int value = 1; };
+template <int R, int... Rs> struct SeqProd<RSeq<R, Rs...>> {
+    static constexpr int value = R * SeqProd<RSeq<Rs...>>::value;
+};
+template <bool B, class A, class C> struct Pick { using type = A; };
+template <class A, class C> struct Pick<false, A, C> { using type = C; };
+// Radix plan -> groups, merging neighbours from the left.
+template <class S, class Acc = GList<>> struct Groups;
+template <class... Gs> struct Groups<RSeq<>, GList<Gs...>> { using type = GList<Gs...>; };
+template <int R, class... Gs> struct Groups<RSeq<R>, GList<Gs...>> { using type = GList<Gs..., RSeq<R>>; };
+template <int R1, int R2, int... Rs, class... Gs> struct Groups<RSeq<R1, R2, Rs...>, GList<Gs...>> {
+    using type = typename Pick<(R1 * R2 <= kMaxGroup), Groups<RSeq<Rs...>, GList<Gs..., RSeq<R1, R2>>>,
+                               Groups<RSeq<R2, Rs...>, GList<Gs..., RSeq<R1>>>>::type::type;
+};
+template <int N> using GroupPlan = typename Groups<typename Plan<N>::type>::type;
+// All but the last group, the last group, and reversal (the groups' order and
+// the radices in each).
+template <class G, class L> struct GCons;
+template <class G, class... Gs> struct GCons<G, GList<Gs...>> { using type = GList<G, Gs...>; };
+template <class L> struct GInit;
+template <class G> struct GInit<GList<G>> { using type = GList<>; };
+template <class G, class G2, class... Gs> struct GInit<GList<G, G2, Gs...>> {
+    using type = typename GCons<G, typename GInit<GList<G2, Gs...>>::type>::type;
+};
+template <class L> struct GLast;
+template <class G> struct GLast<GList<G>> { using type = G; };
+template <class G, class G2, class... Gs> struct GLast<GList<G, G2, Gs...>> {
+    using type = typename GLast<GList<G2, Gs...>>::type;
+};
+template <class L, class Acc = GList<>> struct GRev;
+template <class... As> struct GRev<GList<>, GList<As...>> { using type = GList<As...>; };
+template <class G, class... Gs, class... As> struct GRev<GList<G, Gs...>, GList<As...>> {
+    using type = typename GRev<GList<Gs...>, GList<typename SeqRev<G>::type, As...>>::type;
+};
+
+// The butterflies of one group on its G values, in place (outputs in q order).
+template <int N, int NS, bool INV, int TWS, bool TP, class G> struct GroupRun;
+template <int N, int NS, bool INV, int TWS, bool TP, int R> struct GroupRun<N, NS, INV, TWS, TP, RSeq<R>> {
+    static __device__ __forceinline__ void run(float2* v, int j, const float2* __restrict__ tw) {
+        stage_butterfly<N, NS, R, INV, TWS, TP>(v, j % NS, tw);
+    }
+};
+template <int N, int NS, bool INV, int TWS, bool TP, int R1, int R2>
+struct GroupRun<N, NS, INV, TWS, TP, RSeq<R1, R2>> {
+    static __device__ __forceinline__ void run(float2* v, int j, const float2* __restrict__ tw) {
+        const int k = j % NS;
+        float2 a[R2][R1];
+#pragma unroll
+        for (int p = 0; p < R2; ++p) {
+#pragma unroll
+            for (int r = 0; r < R1; ++r) a[p][r] = v[p + r * R2];
+            stage_butterfly<N, NS, R1, INV, TWS, TP>(a[p], k, tw);
+        }
+#pragma unroll
+        for (int r = 0; r < R1; ++r) {
+            float2 b[R2];
+#pragma unroll
+            for (int p = 0; p < R2; ++p) b[p] = a[p][r];
+            stage_butterfly<N, NS * R1, R2, INV, TWS, TP>(b, k + r * NS, tw);
+#pragma unroll
+            for (int p = 0; p < R2; ++p) v[r + R1 * p] = b[p];
+        }
+    }
+};
+
+// Where element e of line c is in a tile of C lines.  Rows of 8 lines are 64
+// bytes, two to a shared-memory line: which half a row takes flips with bits
+// 3 and 4 of e too, so that two rows 8 or 16 apart (neighbouring outputs of
+// the first group) fall on different banks, as two adjacent rows do.
+template <int C>
+__device__ __forceinline__ int tile_at(int e, int c) {
+    return (C == 8 ? (e ^ (((e >> 3) ^ (e >> 4)) & 1)) : e) * C + c;
+}
+
+// The groups of one transform of the tile's C lines: ld(e, c) gives the
+// inputs, st(e, c, v) takes the outputs; tile holds N C elements.  FROM_TILE /
+// TO_TILE: the first inputs are in the tile / the last outputs go there.
+// Enters with the tile free to be written (unless FROM_TILE: then complete);
+// leaves it synchronised with TO_TILE, else still being read.
+template <int N, int C, int NT, bool INV, int NS, int TWS, bool TP, bool FROM_TILE, bool TO_TILE, class Ld, class St>
+__device__ __forceinline__ void run_groups(float2*, const float2* __restrict__, const Ld&, const St&, GList<>) {}
+
+template <int N, int C, int NT, bool INV, int NS, int TWS, bool TP, bool FROM_TILE, bool TO_TILE, class Ld, class St,
+          class G, class... Gs>
+__device__ __forceinline__ void run_groups(float2* __restrict__ tile, const float2* __restrict__ tw, const Ld& ld,
+                                           const St& st, GList<G, Gs...>) {
+    constexpr int GS = SeqProd<G>::value, NB = N / GS, TOT = NB * C, PER = (TOT + NT - 1) / NT;
+    constexpr bool LAST = sizeof...(Gs) == 0 && !TO_TILE;
+    float2 v[PER][GS];
+#pragma unroll
+    for (int t = 0; t < PER; ++t) {
+        const int b = (int)threadIdx.x + t * NT;
+        if ((TOT % NT) == 0 || b < TOT) {
+            const int c = NT % C == 0 ? (int)threadIdx.x % C : b % C, j = b / C;
+#pragma unroll
+            for (int s = 0; s < GS; ++s) v[t][s] = FROM_TILE ? tile[tile_at<C>(j + s * NB, c)] : ld(j + s * NB, c);
+        }
+    }
+    if (FROM_TILE && !LAST) __syncthreads();
+#pragma unroll
+    for (int t = 0; t < PER; ++t) {
+        const int b = (int)threadIdx.x + t * NT;
+        if ((TOT % NT) == 0 || b < TOT) {
+            const int c = NT % C == 0 ? (int)threadIdx.x % C : b % C, j = b / C;
+            GroupRun<N, NS, INV, TWS, TP, G>::run(v[t], j, tw);
+            const int e0 = (j / NS) * NS * GS + j % NS;
+#pragma unroll
+            for (int q = 0; q < GS; ++q) {
+                if (LAST) st(e0 + q * NS, c, v[t][q]);
+                else tile[tile_at<C>(e0 + q * NS, c)] = v[t][q];
+            }
+        }
+    }
+    if (!LAST) __syncthreads();
+    run_groups<N, C, NT, INV, NS * GS, TWS, TP, true, TO_TILE>(tile, tw, ld, st, GList<Gs...>{});
+}
+
+template <int N, int C, int NT, bool INV, int TWS = 1, bool TP = true, class Ld, class St>
+__device__ __forceinline__ void fft_lines(float2* tile, const float2* __restrict__ tw, const Ld& ld, const St& st) {
+    run_groups<N, C, NT, INV, 1, TWS, TP, false, false>(tile, tw, ld, st, GroupPlan<N>{});
+}
+
+// Forward transform, op(e, c, v) on every mode, inverse transform (as
+// fft_tile_fwd_op_inv, bit for bit): the last forward group's outputs are the
+// first inverse group's inputs, so op and both run on the group's registers.
+template <int N, int C, int NT, int TWS = 1, bool TP = true, class Ld, class St, class F>
+__device__ __forceinline__ void fft_lines_fwd_op_inv(float2* __restrict__ tile, const float2* __restrict__ tw,
+                                                     const Ld& ld, const St& st, const F& op) {
+    using Init = typename GInit<GroupPlan<N>>::type;
+    using G = typename GLast<GroupPlan<N>>::type;
+    using IG = typename SeqRev<G>::type;
+    constexpr int GS = SeqProd<G>::value, NB = N / GS, TOT = NB * C, PER = (TOT + NT - 1) / NT;
+    constexpr bool ONE = NB == 1;  // one group: straight from ld to st
+    run_groups<N, C, NT, false, 1, TWS, TP, false, true>(tile, tw, ld, st, Init{});
+    float2 v[PER][GS];
+#pragma unroll
+    for (int t = 0; t < PER; ++t) {
+        const int b = (int)threadIdx.x + t * NT;
+        if ((TOT % NT) == 0 || b < TOT) {
+            const int c = NT % C == 0 ? (int)threadIdx.x % C : b % C, j = b / C;
+#pragma unroll
+            for (int s = 0; s < GS; ++s) v[t][s] = ONE ? ld(j + s * NB, c) : tile[tile_at<C>(j + s * NB, c)];
+        }
+    }
+    if (!ONE) __syncthreads();
+#pragma unroll
+    for (int t = 0; t < PER; ++t) {
+        const int b = (int)threadIdx.x + t * NT;
+        if ((TOT % NT) == 0 || b < TOT) {
+            const int c = NT % C == 0 ? (int)threadIdx.x % C : b % C, j = b / C;
+            GroupRun<N, NB, false, TWS, TP, G>::run(v[t], j, tw);
+#pragma unroll
+            for (int q = 0; q < GS; ++q) v[t][q] = op(j + q * NB, c, v[t][q]);
+            GroupRun<N, 1, true, TWS, TP, IG>::run(v[t], j, tw);
+#pragma unroll
+            for (int q = 0; q < GS; ++q) {
+                if (ONE) st(j * GS + q, c, v[t][q]);
+                else tile[tile_at<C>(j * GS + q, c)] = v[t][q];
+            }
+        }
+    }
+    if (!ONE) __syncthreads();
+    run_groups<N, C, NT, true, GS, TWS, TP, true, false>(tile, tw, ld, st, typename GRev<Init>::type{});
+}
+
 }  // namespace hgpm

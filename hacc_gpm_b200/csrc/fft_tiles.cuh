@@ -362,6 +362,45 @@ template <int NG> struct XW {
 };
 
 // ---------------------------------------------------------------------------
+// Strided lines (along y or x) in register groups (fft_lines): a tile is C
+// neighbouring columns, C a multiple of 8 (rows of 64 bytes or more), of about
+// ELEMS elements.
+// ---------------------------------------------------------------------------
+template <int NG, int ELEMS> struct LineTile {
+    static constexpr int H = NG / 2;
+    static constexpr int C0 = ELEMS / NG / 8 * 8, C1 = C0 > 32 ? 32 : (C0 < 8 ? 8 : C0);
+    static constexpr int C = C1 > H / 8 * 8 ? H / 8 * 8 : C1;
+    static constexpr int EPT = NG <= 96 ? 8 : 16;  // elements a thread
+    static constexpr int NT0 = (NG * C / EPT + 31) / 32 * 32;
+    static constexpr int NT = NT0 > 512 ? 512 : NT0;
+    static constexpr int MINB = 1024 / NT > 16 ? 16 : 1024 / NT;
+    static constexpr int SMEM = NG * C * 8;
+    // a plane's NG/2 + 1 columns: FULL whole tiles and REM left over, which
+    // go into tiles of their own, PPT planes in each (a tile of one plane's
+    // Nyquist column alone would leave C - 1 of its lines empty)
+    static constexpr int FULL = (H + 1) / C, REM = H + 1 - FULL * C, PPT = REM ? C / REM : 1;
+    static constexpr int TILES = FULL * NG + (REM ? (NG + PPT - 1) / PPT : 0);
+};
+
+// Column c of tile t of a half-spectrum box: its plane, its column; valid.
+template <class T, int NG>
+struct LineCols {
+    int t;
+    __device__ __forceinline__ void at(int c, int& plane, int& col, bool& ok) const {
+        if (t < T::FULL * NG) {
+            plane = t / T::FULL;
+            col = t % T::FULL * T::C + c;
+            ok = true;
+        } else {
+            constexpr int R = T::REM ? T::REM : 1;
+            plane = (t - T::FULL * NG) * T::PPT + c / R;
+            col = T::FULL * T::C + c % R;
+            ok = c / R < T::PPT && plane < NG;
+        }
+    }
+};
+
+// ---------------------------------------------------------------------------
 // host helpers of the launchers
 // ---------------------------------------------------------------------------
 template <class K>
@@ -387,10 +426,6 @@ __global__ void __launch_bounds__(Cfg<NG>::NTX) xfused_kernel(const float2* __re
     const int nvalid = ncols - col0;
     load_tile<NG, C, NT>(tile, in + off, rs, nvalid);
     __syncthreads();
-    if constexpr (Op::kOut == 1) {
-        xone_after_load<NG, NT>(tile, out + off, rs, nvalid, tw, op, iy, col0);
-        return;
-    }
     // the three-output IC pass, whose registers are tight, reads every
     // twiddle from the table
     fft_tile<NG, C, C, false, NT, 1, false>(tile, tw);

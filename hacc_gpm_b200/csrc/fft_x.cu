@@ -6,11 +6,64 @@
 
 namespace hgpm {
 
+// The x pass: forward x transform, the Green's function, inverse x transform
+// of the potential's spectrum, line tiles in register groups.  Bound by issue
+// and latency (at 512^3 before: 138 instructions an element at 63 % of the
+// issue slots, DRAM at 29 %): the quotient of the Green's function (green())
+// takes a third of the instructions a division took, and the tile crosses
+// shared memory 4 times instead of 6 (8 at 1024).  us a pass, against tiles
+// staged through shared memory for every radix and a division per mode: 256^3
+// 52 / 66, 200^3 33 / 43, 512^3 395 / 430, 1024^3 3780 / 4300.
+// Tile size: large enough for 16 columns (whole 128-byte lines) up to 512
+// and 8 above, 2 or more CTAs an SM; small grids take small tiles, so that
+// they spread over the GPU (64^3: 8.7 us in 2^10-element tiles, 10.7 in
+// 2^11); 320 takes 16 columns (104 us; 122 with 8).
 template <int NG>
-__global__ void __launch_bounds__(512, 2) xpot_wide_kernel(const float2* __restrict__ in, float2* __restrict__ out,
-                                                           int ncols, size_t rs, size_t ps,
-                                                           const float2* __restrict__ tw, PotentialOp op) {
-    xone_body<NG, 512, PotentialOp, XW<NG>::C>(in, out, ncols, rs, ps, tw, op, blockIdx.x, blockIdx.y);
+using XT = LineTile<NG, NG <= 64 ? 1024 : NG <= 128 ? 2048 : NG <= 256 ? 4096 : NG < 384 ? 6144 : 8192>;
+
+template <int NG>
+__global__ void __launch_bounds__(XT<NG>::NT, XT<NG>::MINB) xpot_kernel(const float2* __restrict__ in,
+                                                                        float2* __restrict__ out, int zs,
+                                                                        const float2* __restrict__ tw, PotentialOp op,
+                                                                        Slots sl) {
+    using T = XT<NG>;
+    if (slot_idle(sl, blockIdx.y)) return;
+    in += (size_t)blockIdx.y * sl.s0;
+    out += (size_t)blockIdx.y * sl.s1;
+    const LineCols<T, NG> cols{(int)blockIdx.x};
+    const size_t rs = (size_t)NG * zs;
+    fft_lines_fwd_op_inv<NG, T::C, T::NT>(
+        reinterpret_cast<float2*>(hgpm_smem), tw,
+        [&](int e, int c) {
+            int iy, iz;
+            bool ok;
+            cols.at(c, iy, iz, ok);
+            return ok ? __ldcs(in + (size_t)e * rs + (size_t)iy * zs + iz) : make_float2(0.f, 0.f);
+        },
+        [&](int e, int c, float2 v) {
+            int iy, iz;
+            bool ok;
+            cols.at(c, iy, iz, ok);
+            if (ok) __stcs(out + (size_t)e * rs + (size_t)iy * zs + iz, v);
+        },
+        [&](int ix, int c, float2 v) {
+            int iy, iz;
+            bool ok;
+            cols.at(c, iy, iz, ok);
+            if (!ok) iy = iz = 0;  // an empty line of zeros
+            return op.apply(__ldg(&op.cosq[ix]), __ldg(&op.cosq[iy]) + __ldg(&op.cosq[iz]), v);
+        });
+}
+
+template <int NG>
+static cudaError_t xpot_impl(const float2* in, float2* out, int zs, const float2* tw, const PotentialOp& op,
+                             cudaStream_t s, const Slots& sl, int nslots) {
+    using T = XT<NG>;
+    auto k = xpot_kernel<NG>;
+    cudaError_t e = ensure_smem(k, T::SMEM);
+    if (e != cudaSuccess) return e;
+    k<<<dim3(T::TILES, nslots), T::NT, T::SMEM, s>>>(in, out, zs, tw, op, sl);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -111,36 +164,12 @@ cudaError_t launch_gradient(int ng, const float* phi, float4* f, cudaStream_t s,
     return cudaGetLastError();
 }
 
-cudaError_t launch_xpotential(int ng, const float2* in, float2* out, int ncols, size_t rs, size_t ps, int nplanes,
-                              const float2* tw, const double* cosq, double coeff, cudaStream_t s, const Slots& sl,
-                              int nslots) {
+cudaError_t launch_xpotential(int ng, const float2* in, float2* out, int zs, const float2* tw, const double* cosq,
+                              double coeff, cudaStream_t s, const Slots& sl, int nslots) {
     PotentialOp op{cosq, coeff};
     switch (ng) {
 #define X(n) \
-    case n: return xfused_impl<n, PotentialOp>(in, out, ncols, rs, ps, nplanes, 0, tw, op, s, sl, nslots);
-        HGPM_SIZES(X)
-#undef X
-    }
-    return cudaErrorInvalidValue;
-}
-
-template <int NG>
-static cudaError_t xpot_wide_impl(const float2* in, float2* out, int ncols, size_t rs, size_t ps, int nplanes,
-                                  const float2* tw, const PotentialOp& op, cudaStream_t s) {
-    constexpr int C = XW<NG>::C, SMEM = NG * C * 8;
-    auto k = xpot_wide_kernel<NG>;
-    cudaError_t e = ensure_smem(k, SMEM);
-    if (e != cudaSuccess) return e;
-    k<<<dim3(cdiv(ncols, C), nplanes), 512, SMEM, s>>>(in, out, ncols, rs, ps, tw, op);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_xpotential_wide(int ng, const float2* in, float2* out, int ncols, size_t rs, size_t ps, int nplanes,
-                                   const float2* tw, const double* cosq, double coeff, cudaStream_t s) {
-    PotentialOp op{cosq, coeff};
-    switch (ng) {
-#define X(n) \
-    case n: return xpot_wide_impl<n>(in, out, ncols, rs, ps, nplanes, tw, op, s);
+    case n: return xpot_impl<n>(in, out, zs, tw, op, s, sl, nslots);
         HGPM_SIZES(X)
 #undef X
     }

@@ -19,13 +19,32 @@ namespace hgpm {
 // the inverse transform (gradient_kernel: the central difference
 // (phi(x - e_d) - phi(x + e_d)) / 2 multiplies mode k by exactly
 // -i sin(2 pi k_d / ng)).
+// coeff / s rounded to float, 0 for s = 0.  The quotient in double by Newton's
+// iteration for the reciprocal (r' = r + r (1 - s r), from a single-precision
+// start) and one correction by the remainder coeff - s q, exact in fused
+// arithmetic (Markstein 1990): 5 fused operations instead of a division's
+// subroutine with its range checks, which s (in [-6, -3e-6] or 0) and coeff
+// (0.5 / ng^3) never need.  The quotient is within an ulp of double, so the
+// float is the division's unless it lies that close to a rounding boundary.
+__device__ __forceinline__ float green(double s, double coeff) {
+    float r0;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"((float)s));
+    double r = (double)r0;
+    r = fma(r, fma(-s, r, 1.0), r);
+    const double q = coeff * r;
+    return s == 0.0 ? 0.f : (float)fma(fma(-s, q, coeff), r, q);
+}
+
 struct PotentialOp {
     static constexpr int kOut = 1;
     const double* cosq;  // cos(k_i) - 1, one entry per grid index
     double coeff;        // 0.5 / ng^3
     __device__ __forceinline__ float2 pre(int ix, int iy, int iz, float2 v) const {
-        const double s = __ldg(&cosq[ix]) + __ldg(&cosq[iy]) + __ldg(&cosq[iz]);
-        const float g = (s == 0.0) ? 0.f : (float)(coeff / s);
+        return apply(__ldg(&cosq[ix]), __ldg(&cosq[iy]) + __ldg(&cosq[iz]), v);
+    }
+    // cx: the x term, cyz: the sum of the y and z terms
+    __device__ __forceinline__ float2 apply(double cx, double cyz, float2 v) const {
+        const float g = green(cx + cyz, coeff);
         // explicit roundings: the product is never contracted into the
         // butterfly arithmetic around it, so every kernel that applies this
         // operator between its transforms gets the same bits

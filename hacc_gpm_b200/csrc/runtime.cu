@@ -770,12 +770,8 @@ extern "C" int hgpm_solve_gradient(hgpm_ctx* c) {
         if (c->xmode == 1)
             CK(launch_xpotential_tma(ng, c->spec, c->fspec, M + 1, c->zs, c->tw_ng, c->cosq, coeff, c->d_err + 1,
                                      c->stream));
-        else if (c->xmode == 2)
-            CK(launch_xpotential_wide(ng, c->spec, c->fspec, M + 1, (size_t)ng * c->zs, (size_t)c->zs, ng, c->tw_ng,
-                                      c->cosq, coeff, c->stream));
         else
-            CK(launch_xpotential(ng, c->spec, c->fspec, M + 1, (size_t)ng * c->zs, (size_t)c->zs, ng, c->tw_ng,
-                                 c->cosq, coeff, c->stream));
+            CK(launch_xpotential(ng, c->spec, c->fspec, c->zs, c->tw_ng, c->cosq, coeff, c->stream));
         count(c, PH_POISSON, 1);
     }
     const bool plane_inv = c->plane && plane_fft_supported(ng) && kick_uses_phi2(c->kick_choice);

@@ -180,9 +180,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) xpotential_tma_kernel(const __gr
         fft_tile_fwd_op_inv<NG, CT, CT, NT, 1, true>(tile, tw, [&](int ix, int c, float2 v) {
             const int iz = col0 + c;
             if (iz >= ncols) return make_float2(0.f, 0.f);
-            const double sum = cosq[ix] + cy + cosq[iz];
-            const float g = (sum == 0.0) ? 0.f : (float)(coeff / sum);
-            return make_float2(__fmul_rn(v.x, g), __fmul_rn(v.y, g));  // as PotentialOp::pre
+            return PotentialOp{nullptr, coeff}.apply(cosq[ix], cy + cosq[iz], v);
         });
         store_rows<NG, CT, NT>(tile, out + (size_t)iy * zs + col0, rs, ncols - col0);
         // the next TMA load into this buffer follows generic-proxy writes

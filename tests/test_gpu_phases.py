@@ -400,3 +400,26 @@ def test_default_deposit_on_each_side_of_its_rule(ng, np_side, monkeypatch):
                 out.append(s.get_density())
     for o in out[1:]:
         assert np.array_equal(out[0], o)
+
+
+@pytest.mark.parametrize("ng,np_side", [(16, 16), (24, 24), (40, 40), (48, 48), (120, 120), (160, 80), (200, 200),
+                                        (240, 120), (320, 160), (400, 200), (480, 240), (640, 160), (768, 192),
+                                        (800, 200), (960, 240), (1000, 200), (1024, 128)])
+def test_x_pass_line_tiles_equal_tma(ng, np_side, monkeypatch):
+    """The x pass in line tiles (whole tiles, and the left-over columns of
+    several planes in one) and the TMA-fed one move the particles alike, bit
+    for bit, at the grid sides of every tile size."""
+    rng = np.random.default_rng(ng)
+    x = rng.random((np_side ** 3, 3), dtype=np.float32) * np.float32(ng * (1 - 2 ** -20))
+    v = rng.standard_normal((np_side ** 3, 3), dtype=np.float32)
+    out = []
+    for flag in ("1", "2"):
+        monkeypatch.setenv("HGPM_XTMA", flag)
+        with make(ng, np_side) as s:
+            s.load_state(x, v)
+            s.cic()
+            s.solve_gradient()
+            s.kick_drift(0.0123, 1.7, 0.3, 0.25, 2)
+            out.append(s.store_state())
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    assert not np.array_equal(out[0][1], v)
