@@ -52,28 +52,6 @@ __device__ __forceinline__ void split_axis(float x, int ng, int& i, float& o) {
     i = wrap_axis((int)fl, ng);
 }
 
-// State conversion between the reference layout (float3, lattice order) and
-// the internal SoA in Lagrangian-block order (hgpm_device.cuh).
-__global__ void load_state_kernel(const float* __restrict__ x, const float* __restrict__ v, ParticleSoA p,
-                                  int np_side, int B, int ng) {
-    const size_t n = (size_t)np_side * np_side * np_side;
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const size_t q = lattice_of_internal(i, np_side, B);
-    int ix, iy, iz;
-    float ox, oy, oz;
-    split_axis(x[3 * q + 0], ng, ix, ox);
-    split_axis(x[3 * q + 1], ng, iy, oy);
-    split_axis(x[3 * q + 2], ng, iz, oz);
-    p.cell[i] = pack_cell(ix, iy, iz);
-    p.ox[i] = ox;
-    p.oy[i] = oy;
-    p.oz[i] = oz;
-    p.vx[i] = v[3 * q + 0];
-    p.vy[i] = v[3 * q + 1];
-    p.vz[i] = v[3 * q + 2];
-}
-
 // x = cell + offset in float; a sum that rounds up to ng is stored as 0, so
 // positions stay in [0, ng) as the reference's fmod keeps them.
 __device__ __forceinline__ float join_axis(int cell, float o, float fng) {
@@ -81,35 +59,162 @@ __device__ __forceinline__ float join_axis(int cell, float o, float fng) {
     return x >= fng ? x - fng : x;
 }
 
-__global__ void store_state_kernel(ParticleSoA p, float* __restrict__ x, float* __restrict__ v, int np_side, int B,
-                                   int ng) {
-    const size_t n = (size_t)np_side * np_side * np_side;
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const size_t q = lattice_of_internal(i, np_side, B);
-    const uint32_t c = p.cell[i];
-    const float fng = (float)ng;
-    x[3 * q + 0] = join_axis(cell_x(c), p.ox[i], fng);
-    x[3 * q + 1] = join_axis(cell_y(c), p.oy[i], fng);
-    x[3 * q + 2] = join_axis(cell_z(c), p.oz[i], fng);
-    v[3 * q + 0] = p.vx[i];
-    v[3 * q + 1] = p.vy[i];
-    v[3 * q + 2] = p.vz[i];
+// State conversion between the reference layout (float3, lattice order) and
+// the internal SoA in Lagrangian-block order (hgpm_device.cuh).  A warp
+// converts 128 consecutive internal particles, 4 a thread: runs of B
+// z-neighbours, contiguous in both orders, so the float3 side moves as whole
+// float4 (3 a thread and array, passed through shared memory so that
+// neighbouring lanes take neighbouring addresses) and each SoA array as one
+// float4 a thread.  Bound by HBM: 52 bytes a particle each way, 512^3 particles
+// loaded in 1.46 ms and stored in 1.37 a float at a time.  VEC false: the
+// caller's arrays are not 16-byte aligned; 12 floats a thread and array.
+constexpr int kStateThreads = 256;
+
+// Internal index of a run -> its first particle's lattice index.
+template <int B>
+__device__ __forceinline__ unsigned run_lattice(unsigned i, unsigned np, unsigned nb) {
+    constexpr unsigned B3 = B * B * B;
+    const unsigned blk = i / B3, l = i % B3;
+    const unsigned r = blk / nb, bz = blk - r * nb, bx = r / nb, by = r - bx * nb;
+    return ((bx * B + l / (B * B)) * np + by * B + l / B % B) * np + bz * B + l % B;
 }
 
-__global__ void drift_kernel(ParticleSoA p, size_t n, int ng, float pf) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+// The warp's 128 particles' float3 of one array: thread lane gets (IN) or
+// gives (!IN) those of particles 4 lane .. 4 lane + 3 in f[12].
+template <int B, bool IN, bool VEC, class T>
+__device__ __forceinline__ void warp_float3(T* __restrict__ g, float4* __restrict__ buf, unsigned i0, unsigned np,
+                                            unsigned nb, float* __restrict__ f) {
+    const int lane = threadIdx.x & 31;
+    if (!VEC) {
+        T* q = g + 3 * (size_t)run_lattice<B>(i0 + 4 * lane, np, nb);
+#pragma unroll
+        for (int k = 0; k < 12; ++k) {
+            if constexpr (IN) f[k] = __ldg(q + k);
+            else q[k] = f[k];
+        }
+        return;
+    }
+    constexpr int R4 = 3 * B / 4;  // float4 in a run
+    auto at = [&](int k) {
+        const int m = lane + 32 * k;
+        return g + 3 * (size_t)run_lattice<B>(i0 + m / R4 * B, np, nb) + m % R4 * 4;
+    };
+    float4* own = buf + 3 * lane;
+    if constexpr (IN) {
+        float4 v[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[k] = __ldcs(reinterpret_cast<const float4*>(at(k)));
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 3; ++k) buf[lane + 32 * k] = v[k];
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 3; ++k) reinterpret_cast<float4*>(f)[k] = own[k];
+    } else {
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 3; ++k) own[k] = reinterpret_cast<const float4*>(f)[k];
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 3; ++k) __stcs(reinterpret_cast<float4*>(at(k)), buf[lane + 32 * k]);
+    }
+}
+
+template <int B, bool VEC>
+__global__ void __launch_bounds__(kStateThreads) load_state_kernel(const float* __restrict__ x,
+                                                                   const float* __restrict__ v, ParticleSoA p,
+                                                                   unsigned np, int ng, unsigned n) {
+    __shared__ float4 buf[2][kStateThreads / 32][96];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned i0 = (blockIdx.x * (kStateThreads / 32) + warp) * 128u;
+    if (i0 >= n) return;  // whole warps: n is a multiple of 512
+    const unsigned nb = np / B;
+    alignas(16) float xf[12], vf[12];
+    warp_float3<B, true, VEC>(x, buf[0][warp], i0, np, nb, xf);
+    warp_float3<B, true, VEC>(v, buf[1][warp], i0, np, nb, vf);
+    alignas(16) uint32_t c[4];
+    alignas(16) float o[3][4], w[3][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        int i[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            split_axis(xf[3 * k + a], ng, i[a], o[a][k]);
+            w[a][k] = vf[3 * k + a];
+        }
+        c[k] = pack_cell(i[0], i[1], i[2]);
+    }
+    const size_t i = i0 + 4 * lane;
+    float* of[3] = {p.ox, p.oy, p.oz};
+    float* vo[3] = {p.vx, p.vy, p.vz};
+    *reinterpret_cast<uint4*>(p.cell + i) = *reinterpret_cast<uint4*>(c);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        *reinterpret_cast<float4*>(of[a] + i) = *reinterpret_cast<float4*>(o[a]);
+        *reinterpret_cast<float4*>(vo[a] + i) = *reinterpret_cast<float4*>(w[a]);
+    }
+}
+
+template <int B, bool VEC>
+__global__ void __launch_bounds__(kStateThreads) store_state_kernel(ParticleSoA p, float* __restrict__ x,
+                                                                    float* __restrict__ v, unsigned np, int ng,
+                                                                    unsigned n) {
+    __shared__ float4 buf[2][kStateThreads / 32][96];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned i0 = (blockIdx.x * (kStateThreads / 32) + warp) * 128u;
+    if (i0 >= n) return;
+    const unsigned nb = np / B;
+    const size_t i = i0 + 4 * lane;
+    const float* of[3] = {p.ox, p.oy, p.oz};
+    const float* vo[3] = {p.vx, p.vy, p.vz};
+    alignas(16) uint32_t c[4];
+    alignas(16) float o[3][4], w[3][4];
+    *reinterpret_cast<uint4*>(c) = *reinterpret_cast<const uint4*>(p.cell + i);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        *reinterpret_cast<float4*>(o[a]) = *reinterpret_cast<const float4*>(of[a] + i);
+        *reinterpret_cast<float4*>(w[a]) = *reinterpret_cast<const float4*>(vo[a] + i);
+    }
+    const float fng = (float)ng;
+    alignas(16) float xf[12], vf[12];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        xf[3 * k + 0] = join_axis(cell_x(c[k]), o[0][k], fng);
+        xf[3 * k + 1] = join_axis(cell_y(c[k]), o[1][k], fng);
+        xf[3 * k + 2] = join_axis(cell_z(c[k]), o[2][k], fng);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) vf[3 * k + a] = w[a][k];
+    }
+    warp_float3<B, false, VEC>(x, buf[0][warp], i0, np, nb, xf);
+    warp_float3<B, false, VEC>(v, buf[1][warp], i0, np, nb, vf);
+}
+
+// 4 particles a thread (n is a multiple of 512): 44 bytes a particle at HBM
+// rate; 1.22 ms at 512^3 one particle a thread.
+__global__ void __launch_bounds__(256) drift_kernel(ParticleSoA p, size_t n, int ng, float pf) {
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i >= n) return;
-    const uint32_t c = p.cell[i];
-    int ix = cell_x(c), iy = cell_y(c), iz = cell_z(c);
-    float ox = p.ox[i], oy = p.oy[i], oz = p.oz[i];
-    drift_axis(ix, ox, p.vx[i], pf, ng);
-    drift_axis(iy, oy, p.vy[i], pf, ng);
-    drift_axis(iz, oz, p.vz[i], pf, ng);
-    p.cell[i] = pack_cell(ix, iy, iz);
-    p.ox[i] = ox;
-    p.oy[i] = oy;
-    p.oz[i] = oz;
+    alignas(16) uint32_t c[4];
+    alignas(16) float o[3][4], v[3][4];
+    float* of[3] = {p.ox, p.oy, p.oz};
+    const float* vo[3] = {p.vx, p.vy, p.vz};
+    *reinterpret_cast<uint4*>(c) = *reinterpret_cast<const uint4*>(p.cell + i);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        *reinterpret_cast<float4*>(o[a]) = *reinterpret_cast<const float4*>(of[a] + i);
+        *reinterpret_cast<float4*>(v[a]) = *reinterpret_cast<const float4*>(vo[a] + i);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        int ix = cell_x(c[k]), iy = cell_y(c[k]), iz = cell_z(c[k]);
+        drift_axis(ix, o[0][k], v[0][k], pf, ng);
+        drift_axis(iy, o[1][k], v[1][k], pf, ng);
+        drift_axis(iz, o[2][k], v[2][k], pf, ng);
+        c[k] = pack_cell(ix, iy, iz);
+    }
+    *reinterpret_cast<uint4*>(p.cell + i) = *reinterpret_cast<uint4*>(c);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) *reinterpret_cast<float4*>(of[a] + i) = *reinterpret_cast<float4*>(o[a]);
 }
 
 // CICKernel (cic_pm.cu:46-87) with float weights ((w_x*w_y)*w_z)*mass, each
@@ -1558,20 +1663,31 @@ int blocks_per_sm_once(const void* func, int threads, int smem) {
     return per_sm;
 }
 
+// 16-byte aligned caller arrays move as float4.
+static bool aligned16(const void* a, const void* b) { return ((uintptr_t)a | (uintptr_t)b) % 16 == 0; }
+
+template <class K, class... A>
+static cudaError_t state_launch(K k, unsigned n, cudaStream_t s, A... a) {
+    k<<<nblk(n, 4 * kStateThreads), kStateThreads, 0, s>>>(a..., n);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_load_state(const float* x, const float* v, const ParticleSoA& p, int np_side, int B, int ng,
                               cudaStream_t s) {
-    const size_t n = (size_t)np_side * np_side * np_side;
-    load_state_kernel<<<nblk(n, 256), 256, 0, s>>>(x, v, p, np_side, B, ng);
-    return cudaGetLastError();
+    const unsigned np = (unsigned)np_side, n = np * np * np;  // <= 1024^3
+    if (aligned16(x, v))
+        return state_launch(B == 16 ? load_state_kernel<16, true> : load_state_kernel<8, true>, n, s, x, v, p, np, ng);
+    return state_launch(B == 16 ? load_state_kernel<16, false> : load_state_kernel<8, false>, n, s, x, v, p, np, ng);
 }
 cudaError_t launch_store_state(const ParticleSoA& p, float* x, float* v, int np_side, int B, int ng,
                                cudaStream_t s) {
-    const size_t n = (size_t)np_side * np_side * np_side;
-    store_state_kernel<<<nblk(n, 256), 256, 0, s>>>(p, x, v, np_side, B, ng);
-    return cudaGetLastError();
+    const unsigned np = (unsigned)np_side, n = np * np * np;
+    if (aligned16(x, v))
+        return state_launch(B == 16 ? store_state_kernel<16, true> : store_state_kernel<8, true>, n, s, p, x, v, np, ng);
+    return state_launch(B == 16 ? store_state_kernel<16, false> : store_state_kernel<8, false>, n, s, p, x, v, np, ng);
 }
 cudaError_t launch_drift(const ParticleSoA& p, size_t n, int ng, float pf, cudaStream_t s) {
-    drift_kernel<<<nblk(n, 256), 256, 0, s>>>(p, n, ng, pf);
+    drift_kernel<<<nblk(n, 1024), 256, 0, s>>>(p, n, ng, pf);
     return cudaGetLastError();
 }
 

@@ -423,3 +423,36 @@ def test_x_pass_line_tiles_equal_tma(ng, np_side, monkeypatch):
             out.append(s.store_state())
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
     assert not np.array_equal(out[0][1], v)
+
+
+@pytest.mark.parametrize("np_side,ng", [(32, 32), (40, 40), (64, 32), (24, 48)])
+@pytest.mark.parametrize("off", [0, 1, 3])
+def test_device_state_round_trip_at_any_alignment(np_side, ng, off):
+    """Device float3 arrays at 16-byte aligned and at 4-byte aligned addresses
+    (blocks of 16^3 and 8^3 particles) load and store the same particles, and
+    the floats around them are left alone."""
+    import torch
+
+    n = np_side ** 3
+    rng = np.random.default_rng(off + np_side)
+    x = rng.random((n, 3), dtype=np.float32) * np.float32(ng * (1 - 2 ** -20))
+    v = rng.standard_normal((n, 3), dtype=np.float32)
+    xd, vd, xo, vo = (torch.full((3 * n + 8,), -7.0, device="cuda") for _ in range(4))
+    xd[off:off + 3 * n] = torch.from_numpy(x.reshape(-1)).cuda()
+    vd[off:off + 3 * n] = torch.from_numpy(v.reshape(-1)).cuda()
+    torch.cuda.synchronize()
+    with make(ng, np_side) as s:
+        s.load_state(x, v)
+        xh, vh = s.store_state()
+        cells = s.get_cells()
+        s.load_state_device(xd.data_ptr() + 4 * off, vd.data_ptr() + 4 * off)
+        assert np.array_equal(s.get_cells(), cells)
+        s.store_state_device(xo.data_ptr() + 4 * off, vo.data_ptr() + 4 * off)
+        s.sync()
+    i = np.floor(x).astype(np.int64)
+    assert np.array_equal(cells, (i[:, 0] * ng + i[:, 1]) * ng + i[:, 2])
+    assert np.array_equal(vh, v) and np.abs(xh - x).max() <= np.spacing(np.float32(ng))
+    for got, want in ((xo, xh), (vo, vh)):
+        got = got.cpu().numpy()
+        assert np.array_equal(got[off:off + 3 * n], want.reshape(-1))
+        assert (got[:off] == -7.0).all() and (got[off + 3 * n:] == -7.0).all()
