@@ -77,7 +77,7 @@ struct hgpm_ensemble {
     std::vector<EnsClass> cls;
     bool use_graph = false;
     cudaGraphExec_t exec = nullptr;
-    int kick_choice = 0;   // kick and deposit candidates (HGPM_KICK / HGPM_DEPOSIT)
+    int kick_choice = -1;  // kick and deposit candidates (HGPM_KICK / HGPM_DEPOSIT)
     int dep_choice = -1;
     // hgpm_ens_step as one launch per phase across all classes (multi_class.h)
     // when every class is supported; else one launch per phase per class
@@ -248,6 +248,7 @@ extern "C" int hgpm_ens_create(int nclass, const int* ng, const int* np, const i
         if (nslots[i] <= 0 || nslots[i] > 65535 / 3) return efail(E, HGPM_ERR_ARG, "class %d: bad slot count", i);
     }
     const char* kv = getenv("HGPM_KICK");
+    E->kick_choice = kick_default(np[0], ng[0]);  // the same for every shape
     if (kv && kv[0] >= '0' && kv[0] <= '9' && atoi(kv) < kick_candidates(np[0], ng[0])) E->kick_choice = atoi(kv);
     const char* dv = getenv("HGPM_DEPOSIT");
     if (dv && dv[0] >= '0' && dv[0] <= '9') E->dep_choice = atoi(dv);
@@ -431,9 +432,22 @@ extern "C" int hgpm_ens_release(hgpm_ensemble* E, int ci, int slot) {
 }
 
 // Kernels of one class step: deposit (with its spill pass 2), z forward, y
-// forward, x potential, y inverse, z inverse, gradient, kick, slot advance.
+// forward, x potential, y inverse, z inverse, (gradient,) kick, slot advance.
 static int step_kernels(const hgpm_ensemble* E, const EnsClass& k) {
-    return 7 + (deposit_records(E->dep_choice, k.np, k.ng) ? 2 : 1) + kick_kernels(E->kick_choice, k.np, k.ng);
+    return 6 + (kick_uses_phi(E->kick_choice) ? 0 : 1) + (deposit_records(E->dep_choice, k.np, k.ng, k.nslots) ? 2 : 1) +
+           kick_kernels(E->kick_choice, k.np, k.ng);
+}
+
+// The slots with steps to run are about to hold the potential that form of
+// step leaves: their views form a force grid from its spectrum on demand.
+static void mark_stepped(EnsClass& k, bool pair, bool grid) {
+    for (int s = 0; s < k.nslots; ++s) {
+        hgpm_ctx* v = k.views[s];
+        if (!v || !k.in_use[s] || !k.h_mirror[s]) continue;
+        v->phi2_valid = pair;
+        v->phi_valid = !pair;
+        v->force_valid = grid;
+    }
 }
 
 // All phases of one step for every slot of class k, on stream s.
@@ -461,15 +475,25 @@ static int class_step(hgpm_ensemble* E, EnsClass& k, cudaStream_t s) {
                           Slots{act, k.spec_elems, 3 * k.spec_elems}, S));
     ECK(launch_strided(ng, true, k.fspec, M + 1, (size_t)k.zs, (size_t)ng * k.zs, ng, 0, 1, k.tw_ng, s,
                        Slots{act, 3 * k.spec_elems, 0}, S));
+    // what the kick gathers: the paired potential (in the force grid's space,
+    // as a single context places it), the real one, or the force grid
     float4* f4 = reinterpret_cast<float4*>(k.force);
-    float* phi = reinterpret_cast<float*>(k.fspec + k.spec_elems);  // as a single context places it
-    ECK(launch_zinv(ng, k.fspec, phi, ng * ng, k.zs, 0, 0, 1, 1.0f, k.tw_ng, s,
-                    Slots{act, 3 * k.spec_elems, 6 * k.spec_elems}, S));
-    ECK(launch_gradient(ng, phi, f4, s, Slots{act, 6 * k.spec_elems, k.force_elems / 4}, S));
+    float* phi = reinterpret_cast<float*>(k.fspec + k.spec_elems);
+    size_t kick_stride = k.force_elems / 4;
+    if (kick_uses_phi2(E->kick_choice)) {
+        ECK(launch_zinv_pair(ng, k.fspec, k.force, k.zs, k.tw_ng, s, Slots{act, 3 * k.spec_elems, k.force_elems}, S));
+        phi = k.force;
+        kick_stride = k.force_elems;
+    } else {
+        ECK(launch_zinv(ng, k.fspec, phi, ng * ng, k.zs, 0, 0, 1, 1.0f, k.tw_ng, s,
+                        Slots{act, 3 * k.spec_elems, 6 * k.spec_elems}, S));
+        if (kick_uses_phi(E->kick_choice)) kick_stride = 6 * k.spec_elems;
+        else ECK(launch_gradient(ng, phi, f4, s, Slots{act, 6 * k.spec_elems, k.force_elems / 4}, S));
+    }
     ECK(launch_kick_drift(p, k.np, ng, f4, 0.0, 0.0, 0.f, 0.f, 0, E->kick_choice, k.blkwin,
-                          deposit_records(E->dep_choice, k.np, ng), k.kick_spill, s,
-                          Slots{act, k.part_stride, k.force_elems / 4, k.win_stride},
-                          KickSched{k.d_sched, k.d_step, HGPM_MAX_STEPS}, S));
+                          deposit_records(E->dep_choice, k.np, ng, S), k.kick_spill, s,
+                          Slots{act, k.part_stride, kick_stride, k.win_stride},
+                          KickSched{k.d_sched, k.d_step, HGPM_MAX_STEPS}, S, phi));
     ECK(launch_slots_advance(k.d_active, k.d_step, k.d_nsteps, S, s));
     E->launches += step_kernels(E, k);
     return HGPM_OK;
@@ -584,6 +608,9 @@ extern "C" int hgpm_ens_use_graph(hgpm_ensemble* E, int on) {
 
 extern "C" int hgpm_ens_step(hgpm_ensemble* E, int nsteps) {
     if (!E || nsteps < 0) return HGPM_ERR_ARG;
+    if (nsteps > 0)
+        for (auto& k : E->cls) mark_stepped(k, multi_ok(E) || kick_uses_phi2(E->kick_choice),
+                                            !multi_ok(E) && !kick_uses_phi(E->kick_choice));
     if (E->use_graph) {
         if (!E->exec) {
             // the graph covers every class (idle slots cost one early-exit CTA
@@ -636,6 +663,7 @@ extern "C" int hgpm_ens_step_class(hgpm_ensemble* E, int ci, int nsteps) {
     if (rc) return rc;
     if (nsteps < 0) return efail(E, HGPM_ERR_ARG, "nsteps < 0");
     EnsClass& k = E->cls[ci];
+    if (nsteps > 0) mark_stepped(k, kick_uses_phi2(E->kick_choice), !kick_uses_phi(E->kick_choice));
     ECK(cudaEventRecord(k.setup, E->stream));
     ECK(cudaStreamWaitEvent(k.stream, k.setup, 0));
     if (E->use_graph) {

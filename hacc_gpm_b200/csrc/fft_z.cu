@@ -89,7 +89,10 @@ __global__ void __launch_bounds__(kThreads, 4) zpass_r2c_kernel(void* __restrict
 template <int NG>
 __global__ void __launch_bounds__(kThreads) zpass_c2r_pair_kernel(const float2* __restrict__ in,
                                                                   float* __restrict__ out, int nlines, int zs,
-                                                                  const float2* __restrict__ tw) {
+                                                                  const float2* __restrict__ tw, Slots sl) {
+    if (slot_idle(sl, blockIdx.y)) return;
+    in += (size_t)blockIdx.y * sl.s0;
+    out += (size_t)blockIdx.y * sl.s1;
     zpass_c2r_body<NG, true>(in, out, nlines, zs, 1.0f, tw, blockIdx.x);
 }
 
@@ -137,12 +140,13 @@ static cudaError_t zinv_impl(const float2* in, float* out, int nlines, int zs, s
 }
 
 template <int NG>
-static cudaError_t zinv_pair_impl(const float2* in, float* out, int nlines, int zs, const float2* tw, cudaStream_t s) {
+static cudaError_t zinv_pair_impl(const float2* in, float* out, int nlines, int zs, const float2* tw, cudaStream_t s,
+                                  const Slots& sl, int nslots) {
     using G = Cfg<NG>;
     auto k = zpass_c2r_pair_kernel<NG>;
     cudaError_t e = ensure_smem(k, G::ZSMEM);
     if (e != cudaSuccess) return e;
-    k<<<cdiv(nlines, G::L), kThreads, G::ZSMEM, s>>>(in, out, nlines, zs, tw);
+    k<<<dim3(cdiv(nlines, G::L), nslots), kThreads, G::ZSMEM, s>>>(in, out, nlines, zs, tw, sl);
     return cudaGetLastError();
 }
 
@@ -179,10 +183,11 @@ cudaError_t launch_zinv(int ng, const float2* in, float* out, int nlines, int zs
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_zinv_pair(int ng, const float2* in, float* out, int zs, const float2* tw, cudaStream_t s) {
+cudaError_t launch_zinv_pair(int ng, const float2* in, float* out, int zs, const float2* tw, cudaStream_t s,
+                             const Slots& sl, int nslots) {
     switch (ng) {
 #define X(n) \
-    case n: return zinv_pair_impl<n>(in, out, n * n, zs, tw, s);
+    case n: return zinv_pair_impl<n>(in, out, n * n, zs, tw, s, sl, nslots);
         HGPM_SIZES(X)
 #undef X
     }

@@ -49,9 +49,10 @@ cudaError_t launch_zinv(int ng, const float2* in, float* out, int nlines, int zs
 // Unnormalised 3D complex-to-complex FFT of a [ng][ng][ng] float2 grid (z
 // fastest), in place; tw: the ng-point table exp(-2 pi i k / ng).
 cudaError_t launch_fft_c2c(int ng, float2* data, bool inv, const float2* tw, cudaStream_t s);
-// The C2R z pass of one box writing the paired potential (2 ng^3 floats:
+// The C2R z pass writing the paired potential (2 ng^3 floats:
 // cell z of a line holds (phi(z), phi(z+1 mod ng))).
-cudaError_t launch_zinv_pair(int ng, const float2* in, float* out, int zs, const float2* tw, cudaStream_t s);
+cudaError_t launch_zinv_pair(int ng, const float2* in, float* out, int zs, const float2* tw, cudaStream_t s,
+                             const Slots& sl = Slots{}, int nslots = 1);
 // The z and y passes of one box with a thread-block cluster per x plane
 // (sides in HGPM_PLANE_SIZES): the forward R2C z + y passes of the int64
 // density (zeroed) into the half spectrum, and the inverse y + C2R z passes
@@ -121,10 +122,10 @@ bool kick_uses_phi2(int choice);
 // Deposit configurations (bit-identical int64 grids): how many, and the
 // default (used when the choice is -1).
 int deposit_candidates(int np_side, int ng);
-int deposit_default(int np_side, int ng);
+int deposit_default(int np_side, int ng, int nslots = 1);
 // Whether candidate `choice` writes the blocks' window records and launches a
 // spill pass (all but the direct one).
-bool deposit_records(int choice, int np_side, int ng);
+bool deposit_records(int choice, int np_side, int ng, int nslots = 1);
 // Built-in kick candidate (without tuning): the paired potential for 16^3
 // blocks, the real potential for 8^3 blocks.
 int kick_default(int np_side, int ng);

@@ -1839,12 +1839,14 @@ static int deposit_candidates(int cap_default, bool w32, DepositCfg* out) {
 // windows span twice the block) the 32-bit 256-thread kernel with 13312-cell
 // windows (6.9 ms for 512^3 particles on a 1024^3 grid, against 8.3-11.8 for
 // the other windows), otherwise the column kernel (returned-value wraps 103.6
-// us at 200^3, window-sum check 106.7).
+// us at 200^3, window-sum check 106.7).  A batched launch has the blocks of
+// all its slots.
 template <int B>
-static int deposit_default_choice(int np_side, int ng) {
-    if (B == 16) return np_side <= 96 ? 9 : 8;
-    if (ng > np_side) return np_side <= 128 ? 5 : 1;
-    return np_side <= 64 ? 5 : 4;
+static int deposit_default_choice(int np_side, int ng, int nslots) {
+    const long long blocks = (long long)(np_side / B) * (np_side / B) * (np_side / B) * nslots;
+    if (B == 16) return blocks <= 216 ? 9 : 8;
+    if (ng > np_side) return blocks <= 4096 ? 5 : 1;
+    return blocks <= 512 ? 5 : 4;
 }
 
 template <int B, bool SMALL>
@@ -1853,7 +1855,7 @@ static cudaError_t deposit_impl(const ParticleSoA& p, int np_side, int ng, float
                                 int choice, cudaStream_t s) {
     DepositCfg cands[kDepositCands];
     const int ncand = deposit_candidates<B, SMALL>(cap, mass <= 64.0f, cands);
-    const int mode = choice >= 0 && choice < ncand ? choice : deposit_default_choice<B>(np_side, ng);
+    const int mode = choice >= 0 && choice < ncand ? choice : deposit_default_choice<B>(np_side, ng, nslots);
     const DepositCfg& cfg = cands[mode];
     const DepositFn k = cfg.fn;
     if (!k) {  // direct: n <= 1024^3
@@ -1882,16 +1884,16 @@ static cudaError_t deposit_impl(const ParticleSoA& p, int np_side, int ng, float
     return cudaGetLastError();
 }
 
-bool deposit_records(int choice, int np_side, int ng) {
-    if (choice < 0 || choice >= deposit_candidates(np_side, ng)) choice = deposit_default(np_side, ng);
+bool deposit_records(int choice, int np_side, int ng, int nslots) {
+    if (choice < 0 || choice >= deposit_candidates(np_side, ng)) choice = deposit_default(np_side, ng, nslots);
     return choice != (block_side(np_side, ng) == 16 ? 9 : 5);
 }
 
 int deposit_candidates(int np_side, int ng) { return block_side(np_side, ng) == 16 ? kDepositCands : 8; }
 
-int deposit_default(int np_side, int ng) {
-    return block_side(np_side, ng) == 16 ? deposit_default_choice<16>(np_side, ng)
-                                         : deposit_default_choice<8>(np_side, ng);
+int deposit_default(int np_side, int ng, int nslots) {
+    return block_side(np_side, ng) == 16 ? deposit_default_choice<16>(np_side, ng, nslots)
+                                         : deposit_default_choice<8>(np_side, ng, nslots);
 }
 
 cudaError_t launch_deposit(const ParticleSoA& p, int np_side, int ng, float mass, unsigned long long* rho,
