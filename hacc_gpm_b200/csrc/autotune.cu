@@ -218,7 +218,7 @@ extern "C" int hgpm_autotune(hgpm_ctx* c, int reps, int store, int choices[HGPM_
             }, &e);
             CK(e);
         }
-        pick[HGPM_TUNE_YPASS] = hgpm_tune_pick(ms, 2, 1, tol);
+        pick[HGPM_TUNE_YPASS] = hgpm_tune_pick(ms, 2, ypass_tma_default(ng) ? 1 : 0, tol);
         pms[HGPM_TUNE_YPASS] = ms[pick[HGPM_TUNE_YPASS]];
     }
     // x pass with the Green's function: 1 = TMA-fed, 0 and 2 = the line tiles

@@ -9,30 +9,26 @@ namespace hgpm {
 // ---------------------------------------------------------------------------
 // z pass of a complex-to-complex transform of a caller's [ng][ng][ng] grid
 // (forward_fft / backward_fft on a cufftComplex grid, ffts.cu:244-294,
-// 397-445), in place: a CTA transforms CZ<NG> contiguous z lines, staged
-// transposed in shared memory ([m][l], padded) so each stage's butterflies
-// read conflict-free columns.
+// 397-445), in place: a CTA transforms CZ<NG>::L contiguous z lines, 16
+// elements a thread, in register groups (fft_rows).
 template <int NG> struct CZ {
-    static constexpr int L = NG >= 1024 ? 8 : (NG >= 512 ? 16 : (NG >= 128 ? 32 : 64));
-    static constexpr int SMEM = NG * (L + 1) * 8;
+    static constexpr int L0 = 4096 / NG, L = L0 > 32 ? 32 : L0;  // lines a CTA
+    static constexpr int NT0 = (NG * L / 16 + 31) / 32 * 32, NT = NT0;
+    static constexpr int SMEM = L * RowTile<NG>::LS * 8;
 };
 
 template <int NG, bool INV>
-__global__ void __launch_bounds__(kThreads) zpass_c2c_kernel(float2* __restrict__ data, int nlines,
-                                                             const float2* __restrict__ tw) {
-    constexpr int L = CZ<NG>::L, ES = L + 1;
-    float2* buf = reinterpret_cast<float2*>(hgpm_smem);
+__global__ void __launch_bounds__(CZ<NG>::NT, 1024 / CZ<NG>::NT > 16 ? 16 : 1024 / CZ<NG>::NT)
+    zpass_c2c_kernel(float2* __restrict__ data, int nlines, const float2* __restrict__ tw) {
+    constexpr int L = CZ<NG>::L;
     const int line0 = blockIdx.x * L;
-    for (int i = threadIdx.x; i < L * NG; i += kThreads) {
-        const int l = i / NG, m = i % NG;
-        buf[m * ES + l] = line0 + l < nlines ? data[(size_t)(line0 + l) * NG + m] : make_float2(0.f, 0.f);
-    }
-    __syncthreads();
-    fft_tile<NG, L, ES, INV, kThreads>(buf, tw);
-    for (int i = threadIdx.x; i < L * NG; i += kThreads) {
-        const int l = i / NG, m = i % NG;
-        if (line0 + l < nlines) data[(size_t)(line0 + l) * NG + m] = buf[m * ES + l];
-    }
+    data += (size_t)line0 * NG;
+    fft_rows<NG, L, CZ<NG>::NT, INV>(
+        reinterpret_cast<float2*>(hgpm_smem), tw,
+        [&](int l, int e) { return line0 + l < nlines ? __ldcs(data + l * NG + e) : make_float2(0.f, 0.f); },
+        [&](int l, int e, float2 v) {
+            if (line0 + l < nlines) __stcs(data + l * NG + e, v);
+        });
 }
 
 template <int NG>
@@ -42,7 +38,7 @@ static cudaError_t c2c_impl(float2* data, bool inv, const float2* tw, cudaStream
     auto kz = inv ? zpass_c2c_kernel<NG, true> : zpass_c2c_kernel<NG, false>;
     cudaError_t e = ensure_smem(kz, CZ<NG>::SMEM);
     if (e != cudaSuccess) return e;
-    kz<<<cdiv(nlines, L), kThreads, CZ<NG>::SMEM, s>>>(data, nlines, tw);
+    kz<<<cdiv(nlines, L), CZ<NG>::NT, CZ<NG>::SMEM, s>>>(data, nlines, tw);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     // y lines (stride ng, planes x at ng^2), then x lines (stride ng^2,

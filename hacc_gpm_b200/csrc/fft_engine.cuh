@@ -498,4 +498,63 @@ __device__ __forceinline__ void fft_lines_fwd_op_inv(float2* __restrict__ tile, 
     run_groups<N, C, NT, true, GS, TWS, TP, true, false>(tile, tw, ld, st, typename GRev<Init>::type{});
 }
 
+// ---- contiguous lines ------------------------------------------------------
+// The groups of L lines that are contiguous in memory, line-major in the tile:
+// lanes walk a line, so ld and st move neighbouring elements and an exchange
+// reads neighbouring words.  The first group's outputs are GS elements apart;
+// one word of padding per 8 (16 after a group of 16) spreads them, and the
+// next groups' runs of NS, over the banks.
+template <int N> struct RowTile {
+    template <class L> struct First;
+    template <class G, class... Gs> struct First<GList<G, Gs...>> { static constexpr int value = SeqProd<G>::value; };
+    static constexpr int PAD = First<GroupPlan<N>>::value >= 16 ? 4 : 3;
+    static constexpr int LS = N + (N >> PAD) + 1;  // elements between lines
+    static __device__ __forceinline__ int at(int l, int e) { return l * LS + e + (e >> PAD); }
+};
+
+template <int N, int L, int NT, bool INV, int NS, int TWS, bool TP, bool FIRST, class Ld, class St>
+__device__ __forceinline__ void run_rows(float2*, const float2* __restrict__, const Ld&, const St&, GList<>) {}
+
+template <int N, int L, int NT, bool INV, int NS, int TWS, bool TP, bool FIRST, class Ld, class St, class G,
+          class... Gs>
+__device__ __forceinline__ void run_rows(float2* __restrict__ tile, const float2* __restrict__ tw, const Ld& ld,
+                                         const St& st, GList<G, Gs...>) {
+    constexpr int GS = SeqProd<G>::value, NB = N / GS, TOT = NB * L, PER = (TOT + NT - 1) / NT;
+    constexpr bool LAST = sizeof...(Gs) == 0;
+    float2 v[PER][GS];
+#pragma unroll
+    for (int t = 0; t < PER; ++t) {
+        const int b = (int)threadIdx.x + t * NT;
+        if ((TOT % NT) == 0 || b < TOT) {
+            const int l = b / NB, j = b % NB;
+#pragma unroll
+            for (int s = 0; s < GS; ++s) v[t][s] = FIRST ? ld(l, j + s * NB) : tile[RowTile<N>::at(l, j + s * NB)];
+        }
+    }
+    if (!FIRST && !LAST) __syncthreads();
+#pragma unroll
+    for (int t = 0; t < PER; ++t) {
+        const int b = (int)threadIdx.x + t * NT;
+        if ((TOT % NT) == 0 || b < TOT) {
+            const int l = b / NB, j = b % NB;
+            GroupRun<N, NS, INV, TWS, TP, G>::run(v[t], j, tw);
+            const int e0 = (j / NS) * NS * GS + j % NS;
+#pragma unroll
+            for (int q = 0; q < GS; ++q) {
+                if (LAST) st(l, e0 + q * NS, v[t][q]);
+                else tile[RowTile<N>::at(l, e0 + q * NS)] = v[t][q];
+            }
+        }
+    }
+    if (!LAST) __syncthreads();
+    run_rows<N, L, NT, INV, NS * GS, TWS, TP, false>(tile, tw, ld, st, GList<Gs...>{});
+}
+
+// L lines in register groups (fft_lines for contiguous lines): ld(l, e), st(l,
+// e, v); tile: L RowTile<N>::LS elements.
+template <int N, int L, int NT, bool INV, int TWS = 1, bool TP = true, class Ld, class St>
+__device__ __forceinline__ void fft_rows(float2* tile, const float2* __restrict__ tw, const Ld& ld, const St& st) {
+    run_rows<N, L, NT, INV, 1, TWS, TP, true>(tile, tw, ld, st, GroupPlan<N>{});
+}
+
 }  // namespace hgpm

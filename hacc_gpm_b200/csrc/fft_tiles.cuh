@@ -366,23 +366,22 @@ template <int NG> struct XW {
 // neighbouring columns, C a multiple of 8 (rows of 64 bytes or more), of about
 // ELEMS elements.
 // ---------------------------------------------------------------------------
-template <int NG, int ELEMS> struct LineTile {
-    static constexpr int H = NG / 2;
+template <int NG, int ELEMS, int NCOL = NG / 2 + 1> struct LineTile {
     static constexpr int C0 = ELEMS / NG / 8 * 8, C1 = C0 > 32 ? 32 : (C0 < 8 ? 8 : C0);
-    static constexpr int C = C1 > H / 8 * 8 ? H / 8 * 8 : C1;
+    static constexpr int C = C1 > NCOL / 8 * 8 ? NCOL / 8 * 8 : C1;
     static constexpr int EPT = NG <= 96 ? 8 : 16;  // elements a thread
     static constexpr int NT0 = (NG * C / EPT + 31) / 32 * 32;
     static constexpr int NT = NT0 > 512 ? 512 : NT0;
     static constexpr int MINB = 1024 / NT > 16 ? 16 : 1024 / NT;
     static constexpr int SMEM = NG * C * 8;
-    // a plane's NG/2 + 1 columns: FULL whole tiles and REM left over, which
-    // go into tiles of their own, PPT planes in each (a tile of one plane's
+    // a plane's NCOL columns: FULL whole tiles and REM left over, which go
+    // into tiles of their own, PPT planes in each (a tile of one plane's
     // Nyquist column alone would leave C - 1 of its lines empty)
-    static constexpr int FULL = (H + 1) / C, REM = H + 1 - FULL * C, PPT = REM ? C / REM : 1;
+    static constexpr int FULL = NCOL / C, REM = NCOL - FULL * C, PPT = REM ? C / REM : 1;
     static constexpr int TILES = FULL * NG + (REM ? (NG + PPT - 1) / PPT : 0);
 };
 
-// Column c of tile t of a half-spectrum box: its plane, its column; valid.
+// Line c of tile t of a box of NG planes: its plane, its column; valid.
 template <class T, int NG>
 struct LineCols {
     int t;

@@ -50,8 +50,8 @@ struct hgpm_ctx {
     bool phi_valid = false;
     bool force_valid = false;
     bool phi2_valid = false;  // the paired potential, in the force grid's space
-    // kernel variants (environment, read at creation): HGPM_NO_TMA=1 selects the
-    // plain strided y passes, HGPM_XTMA=0|1|2 the fused x pass: TMA-fed (1) or
+    // kernel variants (environment, read at creation): HGPM_NO_TMA=1|0 selects the
+    // line-tile / the TMA-fed y passes (default: ypass_tma_default), HGPM_XTMA=0|1|2 the fused x pass: TMA-fed (1) or
     // in line tiles (0 and 2, the default).  The deposit and kick candidates
     // (bit-identical results) are chosen by the autotuner (hgpm_autotune, or
     // its cache), else HGPM_DEPOSIT / HGPM_KICK, else the built-in defaults.

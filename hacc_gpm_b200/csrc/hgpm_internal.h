@@ -87,6 +87,8 @@ cudaError_t launch_xpk(int ng, const float2* in, int ncols, size_t rs, size_t ps
 // lines when isx); err is set if a bounded mbarrier wait times out.
 cudaError_t launch_strided_tma(int ng, bool inv, bool isx, float2* data, int ncols, int zs, size_t cs, int ncomp,
                                const float2* tw, int* err, cudaStream_t s);
+// Whether a context's y passes are TMA-fed unless chosen otherwise.
+bool ypass_tma_default(int ng);
 // A bounded mbarrier wait that nothing completes (tests of the time-out
 // path): sets *err after `polls` polls.
 cudaError_t launch_wait_timeout_probe(int* err, unsigned polls, cudaStream_t s);

@@ -379,7 +379,7 @@ extern "C" int hgpm_create(const hgpm_params* p, int device, hgpm_ctx** out) {
     c->ncell = (size_t)c->ng * c->ng * c->ng;
     {
         const char* nt = getenv("HGPM_NO_TMA");
-        c->tma = !(nt && nt[0] == '1');
+        c->tma = nt && nt[0] ? nt[0] != '1' : ypass_tma_default(c->ng);
         const char* xt = getenv("HGPM_XTMA");
         if (xt && xt[0] >= '0' && xt[0] <= '2') c->xmode = xt[0] - '0';
         const char* pv = getenv("HGPM_PLANE");

@@ -334,7 +334,7 @@ int hgpm_cic_density_noalloc(const float* x_dev, int np_side, int ng, float* rho
  * results and differ only in speed:
  *   HGPM_TUNE_DEPOSIT  deposit window kernel / CTA shape / window cap,
  *   HGPM_TUNE_KICK     kick gather scheme / CTA shape / units per CTA turn,
- *   HGPM_TUNE_YPASS    1 = TMA-fed persistent y pass, 0 = plain strided,
+ *   HGPM_TUNE_YPASS    1 = TMA-fed persistent y pass, 0 = in line tiles,
  *   HGPM_TUNE_XPASS    2 (the default) and 0 = x pass in line tiles, 1 =
  *                      TMA-fed persistent.
  * hgpm_autotune times every candidate `reps` times on the context's current

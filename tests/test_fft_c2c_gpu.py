@@ -38,3 +38,18 @@ def test_c2c_round_trip_and_legacy_stream():
     assert np.abs(back - a).max() < 2e-5 * np.abs(a).max()
     with pytest.raises(binding.HgpmError):
         binding.fft_c2c(d.data_ptr(), 56, False)
+
+
+@pytest.mark.parametrize("ng", [80, 120, 128, 160, 200, 240, 256, 320, 384, 400, 480, 512])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_c2c_line_tiles_match_float64(ng, inverse):
+    """Every tile size of the z, y and x lines against torch's complex128
+    transform, within the bound of the smaller sides."""
+    g = torch.Generator(device="cuda").manual_seed(ng)
+    d = torch.complex(*(torch.randn(ng, ng, ng, device="cuda", generator=g) for _ in range(2)))
+    a = d.to(torch.complex128)
+    s = torch.cuda.current_stream()
+    binding.fft_c2c(d.data_ptr(), ng, inverse, s.cuda_stream)
+    s.synchronize()
+    ref = torch.fft.ifftn(a, norm="forward") if inverse else torch.fft.fftn(a)
+    assert (d - ref).abs().max() < 2e-5 * ref.abs().max()

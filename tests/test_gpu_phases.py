@@ -456,3 +456,26 @@ def test_device_state_round_trip_at_any_alignment(np_side, ng, off):
         got = got.cpu().numpy()
         assert np.array_equal(got[off:off + 3 * n], want.reshape(-1))
         assert (got[:off] == -7.0).all() and (got[off + 3 * n:] == -7.0).all()
+
+
+@pytest.mark.parametrize("ng,np_side", [(16, 16), (24, 24), (40, 40), (120, 120), (160, 80), (200, 200), (240, 120),
+                                        (400, 200), (480, 240), (640, 160), (800, 200), (960, 240), (1000, 200),
+                                        (1024, 128)])
+def test_y_pass_line_tiles_equal_tma(ng, np_side, monkeypatch):
+    """The y passes in line tiles and the TMA-fed ones move the particles
+    alike, bit for bit, at the grid sides of every tile size."""
+    rng = np.random.default_rng(ng)
+    x = rng.random((np_side ** 3, 3), dtype=np.float32) * np.float32(ng * (1 - 2 ** -20))
+    v = np.zeros_like(x)
+    out = []
+    for flag in ("0", "1"):
+        monkeypatch.setenv("HGPM_NO_TMA", flag)
+        with make(ng, np_side) as s:
+            assert s.tuned_choices()["y_pass"] == (1 if flag == "0" else 0)
+            s.load_state(x, v)
+            s.cic()
+            s.solve_gradient()
+            s.kick_drift(0.0123, 1.7, 0.3, 0.25, 2)
+            out.append(s.store_state())
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    assert out[0][1].any()
