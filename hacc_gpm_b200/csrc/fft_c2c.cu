@@ -36,7 +36,7 @@ static cudaError_t c2c_impl(float2* data, bool inv, const float2* tw, cudaStream
     constexpr int L = CZ<NG>::L;
     const int nlines = NG * NG;
     auto kz = inv ? zpass_c2c_kernel<NG, true> : zpass_c2c_kernel<NG, false>;
-    cudaError_t e = ensure_smem(kz, CZ<NG>::SMEM);
+    cudaError_t e = ensure_smem(kz, CZ<NG>::SMEM, CZ<NG>::NT);
     if (e != cudaSuccess) return e;
     kz<<<cdiv(nlines, L), CZ<NG>::NT, CZ<NG>::SMEM, s>>>(data, nlines, tw);
     e = cudaGetLastError();

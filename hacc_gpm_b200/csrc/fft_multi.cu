@@ -126,7 +126,7 @@ cudaError_t mc_launch(const void* kern, MCTable t, const int* units, int threads
         t.u0[k + 1] = t.u0[k] + units[k] * t.c[k].nslots;
     }
     if (t.u0[t.n] == 0) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = smem_attr_once(kern, smem, threads);
     if (e != cudaSuccess) return e;
     void* args[] = {&t};
     return cudaLaunchKernel(kern, dim3(t.u0[t.n]), dim3(threads), args, smem, s);

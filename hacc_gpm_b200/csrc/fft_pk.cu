@@ -134,7 +134,7 @@ static cudaError_t xpk_impl(const float2* in, int ncols, size_t rs, size_t ps, c
     constexpr int NW = kThreads / 32;
     const int smem = NG * G::CX * 8 + NW * a.nbins * 16;
     auto k = xpk_kernel<NG>;
-    cudaError_t e = smem_attr_once((const void*)k, smem);
+    cudaError_t e = smem_attr_once((const void*)k, smem, kThreads);
     if (e != cudaSuccess) return e;
     const int nchunks = cdiv(ncols, G::CX);
     k<<<nparts, kThreads, smem, s>>>(in, ncols, rs, ps, nchunks, tw, a, part_sum, part_cnt);

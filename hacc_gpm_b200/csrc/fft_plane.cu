@@ -181,7 +181,7 @@ template <int NG, int MINB>
 static cudaError_t plane_impl(bool inv, void* a, float2* spec, int zs, double mean, const float2* tw, cudaStream_t s) {
     constexpr int SMEM = PlaneCfg<NG>::SMEM;
     const void* fn = inv ? (const void*)yz_inv_pair_kernel<NG, MINB> : (const void*)zy_fwd_kernel<NG, MINB>;
-    cudaError_t e = smem_attr_once(fn, SMEM);
+    cudaError_t e = smem_attr_once(fn, SMEM, kThreads);
     if (e != cudaSuccess) return e;
     int nclu = plane_clusters_once(fn, SMEM);
     if (nclu < 1 || nclu > NG) nclu = NG;  // one plane per cluster

@@ -63,7 +63,7 @@ static cudaError_t strided_impl(float2* data, size_t rs, size_t ps, size_t cs, i
                                 cudaStream_t s, const Slots& sl, int nslots) {
     using T = YT<NG, ALL>;
     auto k = strided_kernel<NG, INV, ALL>;
-    cudaError_t e = ensure_smem(k, T::SMEM);
+    cudaError_t e = ensure_smem(k, T::SMEM, T::NT);
     if (e != cudaSuccess) return e;
     k<<<dim3(T::TILES, ncomp, nslots), T::NT, T::SMEM, s>>>(data, rs, ps, cs, tw, sl);
     return cudaGetLastError();

@@ -403,8 +403,8 @@ struct LineCols {
 // host helpers of the launchers
 // ---------------------------------------------------------------------------
 template <class K>
-static inline cudaError_t ensure_smem(K kernel, int bytes) {
-    return smem_attr_once((const void*)kernel, bytes);
+static inline cudaError_t ensure_smem(K kernel, int bytes, int threads) {
+    return smem_attr_once((const void*)kernel, bytes, threads);
 }
 
 static inline unsigned cdiv(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }
@@ -452,7 +452,7 @@ static inline cudaError_t xfused_impl(const float2* in, float2* out, int ncols, 
                                int nslots = 1) {
     using G = Cfg<NG>;
     auto k = xfused_kernel<NG, Op>;
-    cudaError_t e = ensure_smem(k, G::XSMEM);
+    cudaError_t e = ensure_smem(k, G::XSMEM, G::NTX);
     if (e != cudaSuccess) return e;
     dim3 grid(cdiv(ncols, G::CX), nplanes, nslots);
     k<<<grid, G::NTX, G::XSMEM, s>>>(in, out, ncols, rs, ps, out_cs, tw, op, sl);

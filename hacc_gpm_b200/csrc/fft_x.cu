@@ -60,7 +60,7 @@ static cudaError_t xpot_impl(const float2* in, float2* out, int zs, const float2
                              cudaStream_t s, const Slots& sl, int nslots) {
     using T = XT<NG>;
     auto k = xpot_kernel<NG>;
-    cudaError_t e = ensure_smem(k, T::SMEM);
+    cudaError_t e = ensure_smem(k, T::SMEM, T::NT);
     if (e != cudaSuccess) return e;
     k<<<dim3(T::TILES, nslots), T::NT, T::SMEM, s>>>(in, out, zs, tw, op, sl);
     return cudaGetLastError();

@@ -115,12 +115,12 @@ static cudaError_t zfwd_impl(void* in, bool fixed, float2* out, int nlines, int 
     const dim3 grid(cdiv(nlines, G::L), nslots);
     if (fixed) {
         auto k = zpass_r2c_kernel<NG, true>;
-        cudaError_t e = ensure_smem(k, G::ZSMEM);
+        cudaError_t e = ensure_smem(k, G::ZSMEM, kThreads);
         if (e != cudaSuccess) return e;
         k<<<grid, kThreads, G::ZSMEM, s>>>(in, out, nlines, zs, mean, tw, sl);
     } else {
         auto k = zpass_r2c_kernel<NG, false>;
-        cudaError_t e = ensure_smem(k, G::ZSMEM);
+        cudaError_t e = ensure_smem(k, G::ZSMEM, kThreads);
         if (e != cudaSuccess) return e;
         k<<<grid, kThreads, G::ZSMEM, s>>>(in, out, nlines, zs, mean, tw, sl);
     }
@@ -132,7 +132,7 @@ static cudaError_t zinv_impl(const float2* in, float* out, int nlines, int zs, s
                              int ncomp, float scale, const float2* tw, cudaStream_t s, const Slots& sl, int nslots) {
     using G = Cfg<NG>;
     auto k = zpass_c2r_kernel<NG>;
-    cudaError_t e = ensure_smem(k, G::ZSMEM);
+    cudaError_t e = ensure_smem(k, G::ZSMEM, kThreads);
     if (e != cudaSuccess) return e;
     dim3 grid(cdiv(nlines, G::L), ncomp * nslots);
     k<<<grid, kThreads, G::ZSMEM, s>>>(in, out, nlines, zs, in_cs, out_cs, scale, tw, ncomp, sl);
@@ -144,7 +144,7 @@ static cudaError_t zinv_pair_impl(const float2* in, float* out, int nlines, int 
                                   const Slots& sl, int nslots) {
     using G = Cfg<NG>;
     auto k = zpass_c2r_pair_kernel<NG>;
-    cudaError_t e = ensure_smem(k, G::ZSMEM);
+    cudaError_t e = ensure_smem(k, G::ZSMEM, kThreads);
     if (e != cudaSuccess) return e;
     k<<<dim3(cdiv(nlines, G::L), nslots), kThreads, G::ZSMEM, s>>>(in, out, nlines, zs, tw, sl);
     return cudaGetLastError();

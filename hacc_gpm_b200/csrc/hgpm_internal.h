@@ -30,9 +30,12 @@ struct PkArgs {
 #define HGPM_SIZES_TEXT                                                                                     \
     "16,24,32,40,48,64,80,96,120,128,160,192,200,240,256,320,384,400,480,512,640,768,800,960,1000,1024"
 bool fft_size_supported(int ng);
-// cudaFuncAttributeMaxDynamicSharedMemorySize for `func` on the current
-// device, set once per (device, kernel) rather than before every launch.
-cudaError_t smem_attr_once(const void* func, int bytes);
+// The dynamic shared memory `func` may use (bytes a CTA of `threads`) and the
+// share of its SMs' memory that takes, set once per (device, kernel) rather
+// than before every launch.
+cudaError_t smem_attr_once(const void* func, int bytes, int threads);
+// The largest L1 for a kernel without shared memory, set once likewise.
+cudaError_t l1_attr_once(const void* func);
 // Resident CTAs per SM of `func` at this block size and shared memory
 // (occupancy query made once per (device, kernel)).
 int blocks_per_sm_once(const void* func, int threads, int smem);

@@ -1633,20 +1633,53 @@ __global__ void place_kernel(const float* __restrict__ s, size_t scomp, Particle
 // ---------------------------------------------------------------------------
 static inline unsigned nblk(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
-cudaError_t smem_attr_once(const void* func, int bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
+// Attributes of `func` on the current device, set once per (device, kernel).
+// Each kernel says how its SMs split their 256 KB: the ones with tiles or
+// windows ask for the shared memory their resident CTAs need and leave the
+// rest to L1, the gathers (l1_attr_once) ask for the most L1.  Left to the
+// default an SM that other streams keep busy stays in the split it has: with
+// three contexts stepping in turn kicks then ran on what L1 the windows leave
+// (11-13 ms instead of 3.4 for 512^3 particles on 1024^3 cells).  A pass of
+// theirs, default / named: four steps of 256^3 3.04 / 2.80 ms, four of 512^3
+// 23.8 / 22.2, two of 512^3 on 1024^3 74.9 / 55.7, phases of 200^3 1.20 / 1.01.
+// (The most shared memory for all of them is no remedy: the FFT passes live
+// on L1 too, x pass 0.51 against 0.39 ms at 512^3.)
+static cudaError_t func_attr_once(const void* func, int bytes, int threads) {
     static std::mutex mu;
     static std::map<std::pair<int, const void*>, int> done;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> g(mu);
-    int& have = done[{dev, func}];
-    if (have >= bytes) return cudaSuccess;
-    e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) have = bytes;
+    auto it = done.find({dev, func});
+    if (it != done.end() && it->second >= bytes) return cudaSuccess;
+    if (bytes > 48 * 1024) {
+        e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return e;
+    }
+    int carveout = cudaSharedmemCarveoutMaxL1;
+    if (bytes > 0) {
+        int per_sm = 0, most = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, threads, bytes);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+        if (e != cudaSuccess) return e;
+        cudaFuncAttributes fa;
+        if ((e = cudaFuncGetAttributes(&fa, func)) != cudaSuccess) return e;
+        // the smallest of the SM's splits that holds them (1 KB a CTA is the
+        // system's), named by a percentage that rounds up to it
+        const int each = (bytes + (int)fa.sharedSizeBytes + 1024 + 127) / 128 * 128;
+        const int splits[] = {8, 16, 32, 64, 100, 132, 164, 196, 228};
+        int k = 0;
+        while (k < 8 && splits[k] * 1024 < per_sm * each) ++k;
+        carveout = splits[k] * 1024 * 100LL / most > 100 ? 100 : (int)(splits[k] * 1024 * 100LL / most);
+    }
+    e = cudaFuncSetAttribute(func, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
+    if (e == cudaSuccess) done[{dev, func}] = bytes;
     return e;
 }
+
+cudaError_t smem_attr_once(const void* func, int bytes, int threads) { return func_attr_once(func, bytes, threads); }
+cudaError_t l1_attr_once(const void* func) { return func_attr_once(func, 0, 0); }
 
 int blocks_per_sm_once(const void* func, int threads, int smem) {
     static std::mutex mu;
@@ -1866,7 +1899,7 @@ static cudaError_t deposit_impl(const ParticleSoA& p, int np_side, int ng, float
     const int nt = cfg.nt;
     cap = cfg.cap;
     const int smem = cap * cfg.cell_bytes;
-    cudaError_t e = smem_attr_once((const void*)k, smem);
+    cudaError_t e = smem_attr_once((const void*)k, smem, nt);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(spill.cnt, 0, sizeof(int) * nslots, s);
     if (e == cudaSuccess && spill.over) e = cudaMemsetAsync(spill.over, 0, sizeof(int) * nslots, s);
@@ -1877,7 +1910,7 @@ static cudaError_t deposit_impl(const ParticleSoA& p, int np_side, int ng, float
     if (e != cudaSuccess) return e;
     constexpr int NTS = B * B * B >= 1024 ? 1024 : B * B * B;
     auto ks = deposit_spill_kernel<B, SMALL, NTS>;
-    e = smem_attr_once((const void*)ks, kBigCap * 8);
+    e = smem_attr_once((const void*)ks, kBigCap * 8, NTS);
     if (e != cudaSuccess) return e;
     const int per_slot = num_sms() / nslots > 1 ? num_sms() / nslots : 1;  // about one CTA per SM in all
     ks<<<dim3(per_slot, nslots), NTS, kBigCap * 8, s>>>(p, np_side, ng, mass, rho, blkwin, spill, sl);
@@ -1981,6 +2014,8 @@ static cudaError_t kick_flat_launch(const ParticleSoA& p, int np_side, int ng, c
                                     const KickSched& ks, int nslots, cudaStream_t s) {
     const int nblocks = (np_side / B) * (np_side / B) * (np_side / B);
     auto kf = kick_flat_nt_kernel<B, NT, R>;
+    cudaError_t e = l1_attr_once((const void*)kf);
+    if (e != cudaSuccess) return e;
     const int resident = num_sms() * blocks_per_sm_once((const void*)kf, NT, 0);
     const int grid = kick_grid(nblocks * (B * B * B / NT) / R, resident, ng > np_side);
     kf<<<dim3(grid, nslots), NT, 0, s>>>(p, ng, f, deltaT, fscal, pf_a, pf_b, ndrift, nblocks, sl, ks);
@@ -1993,6 +2028,8 @@ static cudaError_t kick_phi_launch(const ParticleSoA& p, int np_side, int ng, co
                                    const KickSched& ks, int nslots, cudaStream_t s) {
     const int nblocks = (np_side / B) * (np_side / B) * (np_side / B);
     auto kf = kick_phi_kernel<B, NT, R, PAIR>;
+    cudaError_t e = l1_attr_once((const void*)kf);
+    if (e != cudaSuccess) return e;
     const int resident = num_sms() * blocks_per_sm_once((const void*)kf, NT, 0);
     const int grid = kick_grid(nblocks * (B * B * B / NT) / R, resident, ng > np_side);
     kf<<<dim3(grid, nslots), NT, 0, s>>>(p, ng, phi, deltaT, fscal, pf_a, pf_b, ndrift, nblocks, sl, ks);
@@ -2029,6 +2066,8 @@ static cudaError_t kick_impl(const ParticleSoA& p, int np_side, int ng, const fl
     }
     constexpr int NT = 512;
     auto ksp = kick_spill_kernel<B>;
+    cudaError_t e = l1_attr_once((const void*)ksp);
+    if (e != cudaSuccess) return e;
     // persistent grid of exactly the resident CTAs (no second round)
     const int sp_grid = num_sms() * blocks_per_sm_once((const void*)ksp, 256, 0);
     if (choice != kKickWindowed) {
@@ -2046,7 +2085,7 @@ static cudaError_t kick_impl(const ParticleSoA& p, int np_side, int ng, const fl
     }
     auto k = kick_win4_kernel<B, NT>;
     const int smem = kWin4Cap * 16;
-    cudaError_t e = smem_attr_once((const void*)k, smem);
+    e = smem_attr_once((const void*)k, smem, NT);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(spill.cnt, 0, sizeof(int) * nslots, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(spill.next, 0, sizeof(int) * nslots, s);
@@ -2228,12 +2267,9 @@ __global__ void mc_advance_kernel(const __grid_constant__ MCTable t) {
 
 cudaError_t mc_persistent(const void* kern, MCTable& t, int threads, int smem, cudaStream_t s) {
     if (t.u0[t.n] == 0) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = smem ? smem_attr_once(kern, smem, threads) : l1_attr_once(kern);
     if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
-    if (e != cudaSuccess) return e;
-    int grid = num_sms() * (per_sm > 0 ? per_sm : 1);
+    int grid = num_sms() * blocks_per_sm_once(kern, threads, smem);
     if (grid > t.u0[t.n]) grid = t.u0[t.n];
     void* args[] = {&t};
     return cudaLaunchKernel(kern, dim3(grid), dim3(threads), args, smem, s);
@@ -2267,7 +2303,7 @@ cudaError_t mc_step(const MCTable& base, cudaStream_t s) {
     MCTable td = base;
     td.u0[0] = 0;
     for (int k = 0; k < base.n; ++k) td.u0[k + 1] = td.u0[k] + base.c[k].nblocks * base.c[k].nslots;
-    e = smem_attr_once((const void*)mc_deposit_kernel, kMCDepCap * 4);
+    e = smem_attr_once((const void*)mc_deposit_kernel, kMCDepCap * 4, 256);
     if (e != cudaSuccess) return e;
     {
         void* dargs[] = {&td};
@@ -2277,7 +2313,7 @@ cudaError_t mc_step(const MCTable& base, cudaStream_t s) {
     {
         const int per = num_sms() / nslots > 1 ? num_sms() / nslots : 1;
         auto ks = mc_spill_kernel;
-        e = smem_attr_once((const void*)ks, kBigCap * 8);
+        e = smem_attr_once((const void*)ks, kBigCap * 8, 1024);
         if (e != cudaSuccess) return e;
         ks<<<dim3(per, nslots), 1024, kBigCap * 8, s>>>(base);
         e = cudaGetLastError();

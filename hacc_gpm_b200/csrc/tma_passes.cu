@@ -266,7 +266,7 @@ static cudaError_t tma_impl(bool inv, bool isx, float2* data, int ncols, int zs,
 #define HGPM_TMA_LAUNCH(I, X)                                                                       \
     {                                                                                               \
         auto k = strided_tma_kernel<NG, I, X>;                                                      \
-        e = smem_attr_once((const void*)k, G::SMEM);                                                \
+        e = smem_attr_once((const void*)k, G::SMEM, kTmaThreads);                                         \
         if (e != cudaSuccess) return e;                                                             \
         int grid = g_num_sms * blocks_per_sm_once((const void*)k, kTmaThreads, G::SMEM);           \
         if (grid > ntiles) grid = ntiles;                                                           \
@@ -298,7 +298,7 @@ static cudaError_t xpotential_tma_impl(float2* in, float2* out, int ncols, int z
     const int nchunks = (ncols + G::CT - 1) / G::CT;
     const int ntiles = nchunks * NG;
     auto k = xpotential_tma_kernel<NG, NT>;
-    e = smem_attr_once((const void*)k, SMEM);
+    e = smem_attr_once((const void*)k, SMEM, NT);
     if (e != cudaSuccess) return e;
     int grid = g_num_sms * blocks_per_sm_once((const void*)k, NT, SMEM);
     if (grid > ntiles) grid = ntiles;
