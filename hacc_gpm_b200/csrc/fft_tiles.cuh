@@ -31,14 +31,11 @@ extern __shared__ float4 hgpm_smem[];
 template <int NG> struct Cfg {
     static constexpr int M = NG / 2;                       // complex length of z lines
     static constexpr int L = M >= 512 ? 8 : (M >= 256 ? 16 : (M >= 96 ? 32 : 64));  // z lines per CTA
-    static constexpr int CS = NG >= 768 ? 8 : 16;          // strided-pass columns per CTA
     static constexpr int CX = NG >= 768 ? 4 : (NG >= 384 ? 8 : 16);  // fused x-pass columns
     static constexpr int ZSMEM = M * (L + 1) * 8;
-    static constexpr int SSMEM = NG * CS * 8;
     static constexpr int XSMEM = 2 * NG * CX * 8;
-    // threads per CTA of the strided and fused x passes: 512 halves the
-    // per-thread register staging so two CTAs (32 warps) fit per SM
-    static constexpr int NTS = NG >= 128 ? 512 : 256;
+    // threads per CTA of the fused x pass: 512 halves the per-thread register
+    // staging so two CTAs (32 warps) fit per SM
     static constexpr int NTX = NG >= 128 ? 512 : 256;
 };
 
@@ -299,69 +296,6 @@ __device__ __forceinline__ void zpass_c2r_body(const float2* __restrict__ in, fl
 }
 
 // ---------------------------------------------------------------------------
-// strided pass (y or x lines), in place,
-// blockIdx = (column chunk, plane, slot * ncomp + comp)
-// ---------------------------------------------------------------------------
-// Column chunk bx of plane by of one component of one box, NT threads.
-template <int NG, bool INV, int NT, int C = Cfg<NG>::CS>
-__device__ __forceinline__ void strided_body(float2* __restrict__ data, int ncols, size_t rs, size_t ps,
-                                             const float2* __restrict__ tw, int bx, int by) {
-    float2* tile = reinterpret_cast<float2*>(hgpm_smem);
-    const int col0 = bx * C;
-    float2* g = data + (size_t)by * ps + col0;
-    const int nvalid = ncols - col0;
-    load_tile<NG, C, NT>(tile, g, rs, nvalid);
-    __syncthreads();
-    fft_tile<NG, C, C, INV, NT>(tile, tw);
-    store_tile<NG, C, NT>(tile, g, rs, nvalid);
-}
-
-// ---------------------------------------------------------------------------
-// x pass fused with a k-space operator producing 3 components:
-//   forward x FFT of the (z,y)-transformed tile -> t = op.pre(k, rho_k) ->
-//   out[0] = IFFT_x(op.comp(0, k, t));  T = IFFT_x(t) ->
-//   out[1] = op.comp(1, ky, kz, T), out[2] = op.comp(2, ky, kz, T).
-// The y and z components' operators (e.g. -i sin(k_y)) are constant along an
-// x line, so they commute with the inverse x transform: two inverse FFTs per
-// tile instead of three.
-// plane = ky index, rows = kx index, columns = kz index; blockIdx.z = slot.
-// ---------------------------------------------------------------------------
-// One-output x pass on a loaded tile: forward x FFT, pre() in registers,
-// inverse x FFT, the same stages and arithmetic as xpotential_tma_kernel (bit
-// for bit).
-template <int NG, int NT, class Op, int C = Cfg<NG>::CX>
-__device__ __forceinline__ void xone_after_load(float2* __restrict__ tile, float2* __restrict__ out, size_t rs,
-                                                int nvalid, const float2* __restrict__ tw, const Op& op, int iy,
-                                                int col0) {
-    fft_tile_fwd_op_inv<NG, C, C, NT, 1, true>(tile, tw,
-                                              [&](int ix, int c, float2 v) { return op.pre(ix, iy, col0 + c, v); });
-    store_tile<NG, C, NT>(tile, out, rs, nvalid);
-}
-
-// The one-output x pass of column chunk bx (C columns) of plane (ky) by of
-// one box.
-template <int NG, int NT, class Op, int C = Cfg<NG>::CX>
-__device__ __forceinline__ void xone_body(const float2* __restrict__ in, float2* __restrict__ out, int ncols,
-                                          size_t rs, size_t ps, const float2* __restrict__ tw, const Op& op, int bx,
-                                          int by) {
-    float2* tile = reinterpret_cast<float2*>(hgpm_smem);
-    const int col0 = bx * C;
-    const size_t off = (size_t)by * ps + col0;
-    const int nvalid = ncols - col0;
-    load_tile<NG, C, NT>(tile, in + off, rs, nvalid);
-    __syncthreads();
-    xone_after_load<NG, NT, Op, C>(tile, out + off, rs, nvalid, tw, op, by, col0);
-}
-
-// The Poisson x pass with twice the columns per CTA (one tile in shared
-// memory, 2 CTAs of 512 threads per SM): more columns in flight per SM for
-// the long lines (1024^3: 8 columns of 1024 points against 4).  Columns stay
-// within the grid side (the Green's function indexes its table by column).
-template <int NG> struct XW {
-    static constexpr int C = 2 * Cfg<NG>::CX <= NG ? 2 * Cfg<NG>::CX : Cfg<NG>::CX;
-};
-
-// ---------------------------------------------------------------------------
 // Strided lines (along y or x) in register groups (fft_lines): a tile is C
 // neighbouring columns, C a multiple of 8 (rows of 64 bytes or more), of about
 // ELEMS elements.
@@ -409,6 +343,16 @@ static inline cudaError_t ensure_smem(K kernel, int bytes, int threads) {
 
 static inline unsigned cdiv(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }
 
+// ---------------------------------------------------------------------------
+// x pass fused with a k-space operator producing 3 components:
+//   forward x FFT of the (z,y)-transformed tile -> t = op.pre(k, rho_k) ->
+//   out[0] = IFFT_x(op.comp(0, k, t));  T = IFFT_x(t) ->
+//   out[1] = op.comp(1, ky, kz, T), out[2] = op.comp(2, ky, kz, T).
+// The y and z components' operators (e.g. -i sin(k_y)) are constant along an
+// x line, so they commute with the inverse x transform: two inverse FFTs per
+// tile instead of three.
+// plane = ky index, rows = kx index, columns = kz index; blockIdx.z = slot.
+// ---------------------------------------------------------------------------
 template <int NG, class Op>
 __global__ void __launch_bounds__(Cfg<NG>::NTX) xfused_kernel(const float2* __restrict__ in, float2* __restrict__ out,
                                                               int ncols, size_t rs, size_t ps, size_t out_cs,

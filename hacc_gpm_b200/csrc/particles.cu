@@ -2200,6 +2200,16 @@ __global__ void __launch_bounds__(256, 4) mc_deposit_kernel(const __grid_constan
     int k, slot, blk;
     if (!mc_find(t, blockIdx.x, k, slot, blk)) return;
     const MCClass& c = t.c[k];
+    if (c.np <= 32) {
+        // blocks of half the box's side: their windows reach around most of
+        // it and overflow into the spill pass (24 us a step for it alone), so
+        // these add straight to the grid
+        const ParticleSoA p = offset_soa(c.p, (size_t)slot * c.part_stride + (size_t)blk * 4096);
+        unsigned long long* rho = c.rho64 + (size_t)slot * c.ncell;
+        for (int i = threadIdx.x; i < 4096; i += 256)
+            deposit_global<true>(rho, __ldg(&p.cell[i]), __ldg(&p.ox[i]), __ldg(&p.oy[i]), __ldg(&p.oz[i]), c.mass, c.ng);
+        return;
+    }
     deposit_col_body<16, 4, 1>(offset_soa(c.p, (size_t)slot * c.part_stride), c.np, c.ng, c.mass,
                                c.rho64 + (size_t)slot * c.ncell, kMCDepCap, c.blkwin + (size_t)slot * c.win_stride,
                                c.spill.items + (size_t)slot * c.spill.nblocks, c.spill.cnt + slot,
