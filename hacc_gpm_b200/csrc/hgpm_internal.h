@@ -82,9 +82,9 @@ cudaError_t launch_gradient(int ng, const float* phi, float4* f, cudaStream_t s,
 cudaError_t launch_xic(int n, const float2* in, float2* out, int ncols, size_t rs, size_t ps, int nplanes,
                        size_t out_cs, const float2* tw, const double* table, int nbins, double k_delta,
                        double pkscale, double inv_delta, const float* kf, int* err, cudaStream_t s);
-cudaError_t launch_xpk(int ng, const float2* in, int ncols, size_t rs, size_t ps, const float2* tw, const PkArgs& a,
-                       double* part_sum, unsigned long long* part_cnt, int nparts, double* sum,
-                       unsigned long long* cnt, cudaStream_t s);
+cudaError_t launch_xpk(int ng, const float2* in, int zs, const float2* tw, const PkArgs& a, double* part_sum,
+                       unsigned long long* part_cnt, int nparts, double* sum, unsigned long long* cnt,
+                       cudaStream_t s);
 
 // Persistent TMA-fed strided pass over a half-spectrum buffer (y lines, or x
 // lines when isx); err is set if a bounded mbarrier wait times out.

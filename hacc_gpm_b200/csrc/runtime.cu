@@ -929,7 +929,7 @@ extern "C" int hgpm_power_spectrum_fold(hgpm_ctx* c, int fold, int nbins, int lo
     if (fold > 9) return fail(c, HGPM_ERR_ARG, "fold %d above 9", fold);
     if (nbins > pk_max_bins()) return fail(c, HGPM_ERR_ARG, "nbins %d above %d", nbins, pk_max_bins());
     if (!c->have_state) return fail(c, HGPM_ERR_STATE, "no particle state loaded");
-    const int ng = c->ng, M = ng / 2;
+    const int ng = c->ng;
     if (!c->pk_part) {
         c->pk_nparts = 4 * 148;
         CK(cudaMalloc(&c->pk_part, (size_t)c->pk_nparts * pk_max_bins() * 8));
@@ -972,7 +972,7 @@ extern "C" int hgpm_power_spectrum_fold(hgpm_ctx* c, int fold, int nbins, int lo
     a.nbins = nbins;
     a.log_bins = log_bins;
     a.scale = (1.0f / ((double)ng * ng * ng)) * (rl_scale / ng);
-    CK(launch_xpk(ng, c->spec, M + 1, (size_t)ng * c->zs, (size_t)c->zs, c->tw_ng, a, c->pk_part, c->pk_pcnt,
+    CK(launch_xpk(ng, c->spec, c->zs, c->tw_ng, a, c->pk_part, c->pk_pcnt,
                   c->pk_nparts, c->pk_sum, c->pk_cnt, c->stream));
     count(c, PH_PK, 2);
     std::vector<double> sum(nbins);

@@ -479,3 +479,43 @@ def test_y_pass_line_tiles_equal_tma(ng, np_side, monkeypatch):
             out.append(s.store_state())
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
     assert out[0][1].any()
+
+
+@pytest.mark.parametrize("ng,np_side", [(16, 16), (24, 24), (48, 48), (120, 120), (160, 80), (200, 200), (320, 160),
+                                        (512, 128), (640, 160)])
+@pytest.mark.parametrize("nbins,log_bins", [(7, False), (221, False), (64, True), (1024, True)])
+def test_power_spectrum_bins_equal_double_binning(ng, np_side, nbins, log_bins):
+    """Mode counts at every tile size equal a count whose bins are formed in
+    double for every mode, with few, many, linear and log-spaced bins."""
+    import torch
+
+    x, v = lattice_state(np_side, ng, disp=1.0, seed=ng)
+    with make(ng, np_side) as s:
+        rl = s.params.rl
+        s.load_state(x, v)
+        k, p, n = s.power_spectrum(nbins, log_bins)
+    i = torch.arange(ng, device="cuda")
+    d = 2 * np.pi / rl
+    kf = (torch.where(i > ng // 2 - 1, i - ng, i).double() * d).float()
+    kz = kf[:ng // 2 + 1].clone()
+    s2 = kf[:, None, None] * kf[:, None, None] + kf[None, :, None] * kf[None, :, None]
+    kmag = (s2 + kz[None, None, :] * kz[None, None, :]).sqrt().double()
+    kmax = np.sqrt(3 * ((ng // 2) * (ng // 2) * d * d))
+    if log_bins:
+        fb = torch.log(kmag / d) / (np.log(kmax / d) / nbins)
+    else:
+        fb = (kmag - d) / ((kmax - d) / nbins)
+    w = torch.full_like(kmag, 2.0)
+    w[:, :, 0] = w[:, :, ng // 2] = 1.0
+    w[0, 0, 0] = w[ng // 2, ng // 2, ng // 2] = 0.0
+    b = torch.trunc(torch.nan_to_num(fb, nan=-2.0, neginf=-2.0))
+    w *= (b >= 0) & (b < nbins) & (fb > -1)
+    want = torch.zeros(nbins, dtype=torch.float64, device="cuda")
+    want.index_add_(0, b.clamp(0, nbins - 1).long().reshape(-1), w.reshape(-1))
+    got = torch.from_numpy(n).double().cuda()
+    # a mode whose double quotient is an integer but for its last bits may
+    # round to the other side of it in another order of operations
+    edge = ((fb - fb.round()).abs() < 1e-12 * nbins).double() * (w > 0)
+    assert (got - want).abs().sum() <= 4 * edge.sum()
+    assert n.sum() == int(w.sum())
+    assert np.isfinite(p).all() and (p[n > 0] > 0).all()
