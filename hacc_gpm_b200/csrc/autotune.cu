@@ -204,7 +204,7 @@ extern "C" int hgpm_autotune(hgpm_ctx* c, int reps, int store, int choices[HGPM_
     CK(cudaMemsetAsync(c->rho64, 0, c->ncell * 8, c->stream));
     CK(launch_deposit(c->part, np, ng, mass, c->rho64, c->blkwin, c->dep_spill, c->stream, Slots{}, 1,
                       pick[HGPM_TUNE_DEPOSIT]));
-    CK(launch_zfwd(ng, c->rho64, true, c->spec, ng * ng, c->zs, mean, c->tw_ng, c->stream));
+    CK(launch_zfwd_rho(ng, c->rho64, c->spec, c->zs, mean, c->tw_ng, c->stream));
     // y pass: 1 = TMA-fed, 0 = plain (in place on the spectrum: timing only;
     // the spectrum is rebuilt below)
     {

@@ -468,7 +468,7 @@ static int class_step(hgpm_ensemble* E, EnsClass& k, cudaStream_t s) {
     const int* act = k.d_active;
     ECK(launch_deposit(p, k.np, ng, mass, k.rho64, k.blkwin, k.dep_spill, s,
                        Slots{act, k.part_stride, k.ncell, k.win_stride}, S, E->dep_choice));
-    ECK(launch_zfwd(ng, k.rho64, true, k.spec, ng * ng, k.zs, mean, k.tw_ng, s, Slots{act, k.ncell, k.spec_elems}, S));
+    ECK(launch_zfwd_rho(ng, k.rho64, k.spec, k.zs, mean, k.tw_ng, s, Slots{act, k.ncell, k.spec_elems}, S));
     ECK(launch_strided(ng, false, k.spec, M + 1, (size_t)k.zs, (size_t)ng * k.zs, ng, 0, 1, k.tw_ng, s,
                        Slots{act, k.spec_elems, 0}, S));
     ECK(launch_xpotential(ng, k.spec, k.fspec, k.zs, k.tw_ng, k.cosq, 0.5 / ((double)ng * ng * ng), s,

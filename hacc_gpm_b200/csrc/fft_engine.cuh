@@ -512,15 +512,16 @@ template <int N> struct RowTile {
     static __device__ __forceinline__ int at(int l, int e) { return l * LS + e + (e >> PAD); }
 };
 
-template <int N, int L, int NT, bool INV, int NS, int TWS, bool TP, bool FIRST, class Ld, class St>
+// TO_TILE: the outputs are left in the tile (RowTile<N>::at), synchronised.
+template <int N, int L, int NT, bool INV, int NS, int TWS, bool TP, bool FIRST, bool TO_TILE, class Ld, class St>
 __device__ __forceinline__ void run_rows(float2*, const float2* __restrict__, const Ld&, const St&, GList<>) {}
 
-template <int N, int L, int NT, bool INV, int NS, int TWS, bool TP, bool FIRST, class Ld, class St, class G,
-          class... Gs>
+template <int N, int L, int NT, bool INV, int NS, int TWS, bool TP, bool FIRST, bool TO_TILE, class Ld, class St,
+          class G, class... Gs>
 __device__ __forceinline__ void run_rows(float2* __restrict__ tile, const float2* __restrict__ tw, const Ld& ld,
                                          const St& st, GList<G, Gs...>) {
     constexpr int GS = SeqProd<G>::value, NB = N / GS, TOT = NB * L, PER = (TOT + NT - 1) / NT;
-    constexpr bool LAST = sizeof...(Gs) == 0;
+    constexpr bool LAST = sizeof...(Gs) == 0 && !TO_TILE;
     float2 v[PER][GS];
 #pragma unroll
     for (int t = 0; t < PER; ++t) {
@@ -547,14 +548,18 @@ __device__ __forceinline__ void run_rows(float2* __restrict__ tile, const float2
         }
     }
     if (!LAST) __syncthreads();
-    run_rows<N, L, NT, INV, NS * GS, TWS, TP, false>(tile, tw, ld, st, GList<Gs...>{});
+    run_rows<N, L, NT, INV, NS * GS, TWS, TP, false, TO_TILE>(tile, tw, ld, st, GList<Gs...>{});
 }
 
 // L lines in register groups (fft_lines for contiguous lines): ld(l, e), st(l,
 // e, v); tile: L RowTile<N>::LS elements.
 template <int N, int L, int NT, bool INV, int TWS = 1, bool TP = true, class Ld, class St>
 __device__ __forceinline__ void fft_rows(float2* tile, const float2* __restrict__ tw, const Ld& ld, const St& st) {
-    run_rows<N, L, NT, INV, 1, TWS, TP, true>(tile, tw, ld, st, GroupPlan<N>{});
+    run_rows<N, L, NT, INV, 1, TWS, TP, true, false>(tile, tw, ld, st, GroupPlan<N>{});
+}
+template <int N, int L, int NT, bool INV, int TWS = 1, bool TP = true, class Ld>
+__device__ __forceinline__ void fft_rows_to_tile(float2* tile, const float2* __restrict__ tw, const Ld& ld) {
+    run_rows<N, L, NT, INV, 1, TWS, TP, true, true>(tile, tw, ld, [](int, int, float2) {}, GroupPlan<N>{});
 }
 
 }  // namespace hgpm

@@ -43,8 +43,8 @@ template <int NG> constexpr int kZLines = NG >= 192 ? Cfg<NG>::L / 2 : Cfg<NG>::
 // One unit of each pass for one grid side.
 template <int NG>
 __device__ __forceinline__ void mc_zfwd_unit(const MCClass& c, int slot, int lu) {
-    zpass_r2c_body<NG, true, kZLines<NG>>(c.rho64 + (size_t)slot * c.ncell, c.spec + (size_t)slot * c.spec_elems,
-                                          NG * NG, c.zs, c.mean, c.tw, lu);
+    zpass_rho_body<NG, kZLines<NG>>(c.rho64 + (size_t)slot * c.ncell, c.spec + (size_t)slot * c.spec_elems, NG * NG,
+                                    c.zs, c.mean, c.tw, lu);
 }
 template <int NG, bool INV>
 __device__ __forceinline__ void mc_ypass_unit(const MCClass& c, int slot, int lu) {

@@ -143,58 +143,37 @@ __device__ __forceinline__ void store_tile_comp(const float2* __restrict__ tile,
 }
 
 // ---------------------------------------------------------------------------
-// z pass, forward R2C.  FIX: input is the int64 fixed-point density
-// (value * 2^32); it is converted to float delta = rho - mean in FP64 and the
-// accumulator is zeroed for the next deposit.  Otherwise input is float.
+// z pass, forward R2C, of the int64 fixed-point density: converted to float
+// delta = rho - mean in FP64 and zeroed for the next deposit.
 // ---------------------------------------------------------------------------
-// The CTA's work (line group bx of one box) as a device function: the
-// single-class kernel below and the multi-class pass (mc_zfwd_kernel) run
-// the same code.
-template <int NG, bool FIX, int L = Cfg<NG>::L>
-__device__ __forceinline__ void zpass_r2c_body(void* __restrict__ in_, float2* __restrict__ out, int nlines, int zs,
-                                               double mean, const float2* __restrict__ tw, int bx) {
+// The multi-class pass: the lines of group bx of one box.  (The register groups
+// of z_rho below lose there, 64 against 58 us a step of the five sides.)
+template <int NG, int L>
+__device__ __forceinline__ void zpass_rho_body(unsigned long long* __restrict__ in, float2* __restrict__ out, int nlines,
+                                               int zs, double mean, const float2* __restrict__ tw, int bx) {
     constexpr int M = NG / 2, ES = L + 1;
     float2* buf = reinterpret_cast<float2*>(hgpm_smem);
     const int line0 = bx * L;
     constexpr int TOT = L * M;
     constexpr int PER = (TOT + kThreads - 1) / kThreads;
-    if (FIX) {
-        ulonglong2 q[PER];
+    ulonglong2 q[PER];
 #pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            const int i = threadIdx.x + t * kThreads;
-            const int l = i / M, m = i % M;
-            q[t] = make_ulonglong2(0ull, 0ull);
-            if (((TOT % kThreads) == 0 || i < TOT) && line0 + l < nlines)
-                q[t] = __ldcs(reinterpret_cast<const ulonglong2*>(reinterpret_cast<unsigned long long*>(in_) +
-                                                                  (size_t)(line0 + l) * NG) + m);
-        }
+    for (int t = 0; t < PER; ++t) {
+        const int i = threadIdx.x + t * kThreads;
+        const int l = i / M, m = i % M;
+        q[t] = make_ulonglong2(0ull, 0ull);
+        if (((TOT % kThreads) == 0 || i < TOT) && line0 + l < nlines)
+            q[t] = __ldcs(reinterpret_cast<const ulonglong2*>(in + (size_t)(line0 + l) * NG) + m);
+    }
 #pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            const int i = threadIdx.x + t * kThreads;
-            const int l = i / M, m = i % M;
-            if (((TOT % kThreads) == 0 || i < TOT)) {
-                if (line0 + l < nlines)
-                    __stcs(reinterpret_cast<ulonglong2*>(reinterpret_cast<unsigned long long*>(in_) +
-                                                         (size_t)(line0 + l) * NG) + m, make_ulonglong2(0ull, 0ull));
-                buf[m * ES + l] = make_float2((float)((double)(long long)q[t].x * kFixInv - mean),
-                                              (float)((double)(long long)q[t].y * kFixInv - mean));
-            }
-        }
-    } else {
-        float2 z[PER];
-#pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            const int i = threadIdx.x + t * kThreads;
-            const int l = i / M, m = i % M;
-            z[t] = make_float2(0.f, 0.f);
-            if (((TOT % kThreads) == 0 || i < TOT) && line0 + l < nlines)
-                z[t] = reinterpret_cast<const float2*>(reinterpret_cast<const float*>(in_) + (size_t)(line0 + l) * NG)[m];
-        }
-#pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            const int i = threadIdx.x + t * kThreads;
-            if ((TOT % kThreads) == 0 || i < TOT) buf[(i % M) * ES + i / M] = z[t];
+    for (int t = 0; t < PER; ++t) {
+        const int i = threadIdx.x + t * kThreads;
+        const int l = i / M, m = i % M;
+        if (((TOT % kThreads) == 0 || i < TOT)) {
+            if (line0 + l < nlines)
+                __stcs(reinterpret_cast<ulonglong2*>(in + (size_t)(line0 + l) * NG) + m, make_ulonglong2(0ull, 0ull));
+            buf[m * ES + l] = make_float2((float)((double)(long long)q[t].x * kFixInv - mean),
+                                          (float)((double)(long long)q[t].y * kFixInv - mean));
         }
     }
     __syncthreads();
@@ -219,6 +198,67 @@ __device__ __forceinline__ void zpass_r2c_body(void* __restrict__ in_, float2* _
             dst[M - k] = make_float2(xm.x, -xm.y);
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// R2C z pass: L contiguous lines of NG reals, as NG/2 complex each, in register
+// groups (fft_rows), NT threads.  The first group takes its elements from
+// global memory.
+// ---------------------------------------------------------------------------
+template <int NG, int ELEMS> struct ZTile {
+    static constexpr int M = NG / 2;
+    static constexpr int L0 = ELEMS / M, L = L0 < 1 ? 1 : L0;
+    static constexpr int EPT = NG <= 96 ? 8 : 16;
+    static constexpr int NT0 = (M * L / EPT + 31) / 32 * 32, NT = NT0 < L ? (L + 31) / 32 * 32 : NT0;
+    static constexpr int MINB = 1024 / NT > 16 ? 16 : 1024 / NT;
+    static constexpr int SMEM = L * RowTile<M>::LS * 8;
+};
+
+// R2C of lines [line0, line0 + L): ld(line, m) gives cells (2m, 2m + 1).
+// Leaves the tile being read.
+template <int NG, int L, int NT, class Ld>
+__device__ __forceinline__ void z_r2c(float2* __restrict__ tile, float2* __restrict__ out, int line0, int nlines, int zs,
+                                      const float2* __restrict__ tw, const Ld& ld) {
+    constexpr int M = NG / 2, H = M / 2 + 1;
+    using R = RowTile<M>;
+    fft_rows_to_tile<M, L, NT, false, 2>(tile, tw, [&](int l, int e) {
+        return line0 + l < nlines ? ld(line0 + l, e) : make_float2(0.f, 0.f);
+    });
+    for (int i = threadIdx.x; i < L * H; i += NT) {
+        const int l = i / H, k = i % H;
+        const int line = line0 + l;
+        if (line >= nlines) continue;
+        const float2 zk = tile[R::at(l, k)];
+        const float2 zm = tile[R::at(l, k ? M - k : 0)];
+        const float2 w = __ldg(&tw[k]);
+        // E = (Zk + conj Zm)/2, O = -i (Zk - conj Zm)/2, X[k] = E + w O,
+        // X[M-k] = conj(E - w O)
+        const float2 e = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
+        const float2 o = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
+        const float2 wo = cmul(w, o);
+        float2* dst = out + (size_t)line * zs;
+        dst[k] = cadd(e, wo);
+        if (k != M - k) {
+            const float2 xm = csub(e, wo);
+            dst[M - k] = make_float2(xm.x, -xm.y);
+        }
+    }
+}
+
+// R2C of the int64 fixed-point density less the mean (formed in FP64); the
+// lines are zeroed for the next deposit.
+template <int NG, int L, int NT>
+__device__ __forceinline__ void z_rho(float2* __restrict__ tile, unsigned long long* __restrict__ rho,
+                                      float2* __restrict__ out, int line0, int nlines, int zs, double mean,
+                                      const float2* __restrict__ tw) {
+    z_r2c<NG, L, NT>(tile, out, line0, nlines, zs, tw, [&](int line, int m) {
+        const ulonglong2 q = __ldcs(reinterpret_cast<const ulonglong2*>(rho + (size_t)line * NG) + m);
+        return make_float2((float)((double)(long long)q.x * kFixInv - mean), (float)((double)(long long)q.y * kFixInv - mean));
+    });
+    // every line has been read (the transform's barriers)
+    const int n = (nlines - line0 < L ? nlines - line0 : L) * (NG / 2);
+    ulonglong2* q = reinterpret_cast<ulonglong2*>(rho + (size_t)line0 * NG);
+    for (int i = threadIdx.x; i < n; i += NT) __stcs(q + i, make_ulonglong2(0ull, 0ull));
 }
 
 // ---------------------------------------------------------------------------

@@ -6,84 +6,34 @@
 
 namespace hgpm {
 
-// The single-class kernel: zpass_r2c_body's code with the slot prologue
-// written out (as a kernel with its own restrict-qualified parameters it
-// compiles without the body's 76 bytes of spills at 512^3).
-template <int NG, bool FIX>
-__global__ void __launch_bounds__(kThreads, 4) zpass_r2c_kernel(void* __restrict__ in_, float2* __restrict__ out,
-                                                             int nlines, int zs, double mean,
-                                                             const float2* __restrict__ tw, Slots sl) {
-    constexpr int M = NG / 2, L = Cfg<NG>::L, ES = L + 1;
-    float2* buf = reinterpret_cast<float2*>(hgpm_smem);
+// R2C: tiles of about 4096 elements, 16 a thread, smaller on small grids, so
+// that they spread over the GPU.  At its traffic's HBM time where the line's
+// radices are powers of two (512^3: 0.44 ms for the 20 bytes a cell read,
+// zeroed and written); elsewhere bound by issue, and by spills when it staged a
+// tile at 256 threads whatever the side: us a pass, against that, 200^3 40 / 49,
+// 320^3 134 / 215, 480^3 486 / 818, 768^3 2047 / 3191, 1000^3 4690 / 7378.
+// (The C2R pass loses in this form, 0.40 against 0.28 ms at 512^3: every mode
+// is read twice for the mirrored pairs.)
+template <int NG> using ZT = ZTile<NG, NG <= 32 ? 256 : NG <= 48 ? 512 : NG <= 64 ? 1024 : NG <= 128 ? 2048 : 4096>;
+
+// The density accumulator's z pass, and a real grid's.
+template <int NG>
+__global__ void __launch_bounds__(ZT<NG>::NT, ZT<NG>::MINB)
+    zpass_rho_kernel(unsigned long long* __restrict__ rho, float2* __restrict__ out, int nlines, int zs, double mean, const float2* __restrict__ tw,
+                     Slots sl) {
+    using T = ZT<NG>;
     if (slot_idle(sl, blockIdx.y)) return;
-    // slot stride s0 counts input elements (int64 when FIX, float otherwise)
-    in_ = FIX ? (void*)(reinterpret_cast<unsigned long long*>(in_) + (size_t)blockIdx.y * sl.s0)
-              : (void*)(reinterpret_cast<float*>(in_) + (size_t)blockIdx.y * sl.s0);
-    out += (size_t)blockIdx.y * sl.s1;
-    const int line0 = blockIdx.x * L;
-    constexpr int TOT = L * M;
-    constexpr int PER = (TOT + kThreads - 1) / kThreads;
-    if (FIX) {
-        ulonglong2 q[PER];
-#pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            const int i = threadIdx.x + t * kThreads;
-            const int l = i / M, m = i % M;
-            q[t] = make_ulonglong2(0ull, 0ull);
-            if (((TOT % kThreads) == 0 || i < TOT) && line0 + l < nlines)
-                q[t] = __ldcs(reinterpret_cast<const ulonglong2*>(reinterpret_cast<unsigned long long*>(in_) +
-                                                                  (size_t)(line0 + l) * NG) + m);
-        }
-#pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            const int i = threadIdx.x + t * kThreads;
-            const int l = i / M, m = i % M;
-            if (((TOT % kThreads) == 0 || i < TOT)) {
-                if (line0 + l < nlines)
-                    __stcs(reinterpret_cast<ulonglong2*>(reinterpret_cast<unsigned long long*>(in_) +
-                                                         (size_t)(line0 + l) * NG) + m, make_ulonglong2(0ull, 0ull));
-                buf[m * ES + l] = make_float2((float)((double)(long long)q[t].x * kFixInv - mean),
-                                              (float)((double)(long long)q[t].y * kFixInv - mean));
-            }
-        }
-    } else {
-        float2 z[PER];
-#pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            const int i = threadIdx.x + t * kThreads;
-            const int l = i / M, m = i % M;
-            z[t] = make_float2(0.f, 0.f);
-            if (((TOT % kThreads) == 0 || i < TOT) && line0 + l < nlines)
-                z[t] = reinterpret_cast<const float2*>(reinterpret_cast<const float*>(in_) + (size_t)(line0 + l) * NG)[m];
-        }
-#pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            const int i = threadIdx.x + t * kThreads;
-            if ((TOT % kThreads) == 0 || i < TOT) buf[(i % M) * ES + i / M] = z[t];
-        }
-    }
-    __syncthreads();
-    fft_tile<M, L, ES, false, kThreads, 2>(buf, tw);
-    constexpr int H = M / 2 + 1;
-    for (int i = threadIdx.x; i < L * H; i += kThreads) {
-        const int l = i / H, k = i % H;
-        const int line = line0 + l;
-        if (line >= nlines) continue;
-        const float2 zk = buf[k * ES + l];
-        const float2 zm = buf[((M - k) % M) * ES + l];
-        const float2 w = __ldg(&tw[k]);
-        // E = (Zk + conj Zm)/2, O = -i (Zk - conj Zm)/2, X[k] = E + w O,
-        // X[M-k] = conj(E - w O)
-        const float2 e = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
-        const float2 o = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
-        const float2 wo = cmul(w, o);
-        float2* dst = out + (size_t)line * zs;
-        dst[k] = cadd(e, wo);
-        if (k != M - k) {
-            const float2 xm = csub(e, wo);
-            dst[M - k] = make_float2(xm.x, -xm.y);
-        }
-    }
+    z_rho<NG, T::L, T::NT>(reinterpret_cast<float2*>(hgpm_smem), rho + (size_t)blockIdx.y * sl.s0,
+                           out + (size_t)blockIdx.y * sl.s1, blockIdx.x * T::L, nlines, zs, mean, tw);
+}
+
+template <int NG>
+__global__ void __launch_bounds__(ZT<NG>::NT, ZT<NG>::MINB)
+    zpass_r2c_kernel(const float* __restrict__ in, float2* __restrict__ out, int nlines, int zs,
+                     const float2* __restrict__ tw) {
+    using T = ZT<NG>;
+    z_r2c<NG, T::L, T::NT>(reinterpret_cast<float2*>(hgpm_smem), out, blockIdx.x * T::L, nlines, zs, tw,
+                           [&](int line, int m) { return __ldcs(reinterpret_cast<const float2*>(in + (size_t)line * NG) + m); });
 }
 
 template <int NG>
@@ -109,21 +59,23 @@ __global__ void __launch_bounds__(kThreads) zpass_c2r_kernel(const float2* __res
 }
 
 template <int NG>
-static cudaError_t zfwd_impl(void* in, bool fixed, float2* out, int nlines, int zs, double mean,
-                             const float2* tw, cudaStream_t s, const Slots& sl, int nslots) {
-    using G = Cfg<NG>;
-    const dim3 grid(cdiv(nlines, G::L), nslots);
-    if (fixed) {
-        auto k = zpass_r2c_kernel<NG, true>;
-        cudaError_t e = ensure_smem(k, G::ZSMEM, kThreads);
-        if (e != cudaSuccess) return e;
-        k<<<grid, kThreads, G::ZSMEM, s>>>(in, out, nlines, zs, mean, tw, sl);
-    } else {
-        auto k = zpass_r2c_kernel<NG, false>;
-        cudaError_t e = ensure_smem(k, G::ZSMEM, kThreads);
-        if (e != cudaSuccess) return e;
-        k<<<grid, kThreads, G::ZSMEM, s>>>(in, out, nlines, zs, mean, tw, sl);
-    }
+static cudaError_t zfwd_impl(const float* in, float2* out, int nlines, int zs, const float2* tw, cudaStream_t s) {
+    using T = ZT<NG>;
+    auto k = zpass_r2c_kernel<NG>;
+    cudaError_t e = ensure_smem(k, T::SMEM, T::NT);
+    if (e != cudaSuccess) return e;
+    k<<<cdiv(nlines, T::L), T::NT, T::SMEM, s>>>(in, out, nlines, zs, tw);
+    return cudaGetLastError();
+}
+
+template <int NG>
+static cudaError_t zrho_impl(unsigned long long* rho, float2* out, int zs, double mean, const float2* tw, cudaStream_t s,
+                             const Slots& sl, int nslots) {
+    using T = ZT<NG>;
+    auto k = zpass_rho_kernel<NG>;
+    cudaError_t e = ensure_smem(k, T::SMEM, T::NT);
+    if (e != cudaSuccess) return e;
+    k<<<dim3(cdiv(NG * NG, T::L), nslots), T::NT, T::SMEM, s>>>(rho, out, NG * NG, zs, mean, tw, sl);
     return cudaGetLastError();
 }
 
@@ -161,11 +113,21 @@ bool fft_size_supported(int ng) {
     }
 }
 
-cudaError_t launch_zfwd(int ng, void* in, bool fixed, float2* out, int nlines, int zs, double mean,
-                        const float2* tw, cudaStream_t s, const Slots& sl, int nslots) {
+cudaError_t launch_zfwd(int ng, const float* in, float2* out, int nlines, int zs, const float2* tw, cudaStream_t s) {
     switch (ng) {
 #define X(n) \
-    case n: return zfwd_impl<n>(in, fixed, out, nlines, zs, mean, tw, s, sl, nslots);
+    case n: return zfwd_impl<n>(in, out, nlines, zs, tw, s);
+        HGPM_SIZES(X)
+#undef X
+    }
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_zfwd_rho(int ng, unsigned long long* rho, float2* out, int zs, double mean, const float2* tw,
+                            cudaStream_t s, const Slots& sl, int nslots) {
+    switch (ng) {
+#define X(n) \
+    case n: return zrho_impl<n>(rho, out, zs, mean, tw, s, sl, nslots);
         HGPM_SIZES(X)
 #undef X
     }

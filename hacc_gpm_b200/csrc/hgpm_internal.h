@@ -44,8 +44,11 @@ int pk_max_bins();
 // Launchers of the step's kernels.  `sl`/`nslots` batch the launch over
 // nslots boxes of one size class (Slots in hgpm_device.cuh); the defaults
 // launch one box.
-cudaError_t launch_zfwd(int ng, void* in, bool fixed, float2* out, int nlines, int zs, double mean,
-                        const float2* tw, cudaStream_t s, const Slots& sl = Slots{}, int nslots = 1);
+// The R2C z pass of a real grid, or of the int64 density less the mean (which
+// it leaves zeroed; sl.s0: cells a slot).
+cudaError_t launch_zfwd(int ng, const float* in, float2* out, int nlines, int zs, const float2* tw, cudaStream_t s);
+cudaError_t launch_zfwd_rho(int ng, unsigned long long* rho, float2* out, int zs, double mean, const float2* tw,
+                            cudaStream_t s, const Slots& sl = Slots{}, int nslots = 1);
 cudaError_t launch_zinv(int ng, const float2* in, float* out, int nlines, int zs, size_t in_cs, size_t out_cs,
                         int ncomp, float scale, const float2* tw, cudaStream_t s, const Slots& sl = Slots{},
                         int nslots = 1);

@@ -741,7 +741,7 @@ static int forward_zy(hgpm_ctx* c) {
     }
     {
         PhaseScope ps(c, PH_ZFWD);
-        CK(launch_zfwd(ng, c->rho64, true, c->spec, ng * ng, c->zs, mean_density(c), c->tw_ng, c->stream));
+        CK(launch_zfwd_rho(ng, c->rho64, c->spec, c->zs, mean_density(c), c->tw_ng, c->stream));
         c->rho_dirty = false;
         count(c, PH_ZFWD, 1);
     }
@@ -1092,7 +1092,7 @@ static int ic_common(hgpm_ctx* c, const float* noise_host, const double* table, 
         }
         if ((e = cudaMemsetAsync(c->d_err, 0, 4, c->stream)) != cudaSuccess) { rc = fail(c, HGPM_ERR_CUDA, "%s", cudaGetErrorString(e)); break; }
         const size_t cs = (size_t)n * n * c->zs_np;
-        e = launch_zfwd(n, noise, false, c->spec, n * n, c->zs_np, 0.0, c->tw_np, c->stream);
+        e = launch_zfwd(n, noise, c->spec, n * n, c->zs_np, c->tw_np, c->stream);
         if (e == cudaSuccess) e = launch_strided(n, false, c->spec, M + 1, (size_t)c->zs_np, (size_t)n * c->zs_np, n, 0, 1, c->tw_np, c->stream);
         if (e == cudaSuccess)
             e = launch_xic(n, c->spec, c->fspec, M + 1, (size_t)n * c->zs_np, (size_t)c->zs_np, n, cs, c->tw_np, d_table,

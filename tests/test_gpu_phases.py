@@ -519,3 +519,31 @@ def test_power_spectrum_bins_equal_double_binning(ng, np_side, nbins, log_bins):
     assert (got - want).abs().sum() <= 4 * edge.sum()
     assert n.sum() == int(w.sum())
     assert np.isfinite(p).all() and (p[n > 0] > 0).all()
+
+
+@pytest.mark.parametrize("ng,np_side", [(240, 80), (256, 64), (320, 80), (384, 96), (400, 80), (480, 96), (512, 64),
+                                        (640, 64), (1000, 40)])
+def test_solve_of_large_sides_matches_double_fft(ng, np_side):
+    """Sides beyond the oracle's reach: the forces against a double-precision
+    transform of the same density on the device."""
+    import torch
+
+    x, v = lattice_state(np_side, ng, disp=1.2, seed=ng + 1)
+    with make(ng, np_side) as s:
+        s.load_state(x, v)
+        s.cic()
+        rho = torch.from_numpy(s.get_density()).cuda().double().reshape(ng, ng, ng)
+        s.solve_gradient()
+        f = s.get_force()
+    d = np.float32(2.0 * np.pi / np.float32(ng))  # the oracle's cosine arguments
+    c = torch.from_numpy(np.cos(np.arange(ng).astype(np.float32) * d).astype(np.float64)).cuda()
+    g = 0.5 / (c[:, None, None] + c[None, :, None] + c[None, None, : ng // 2 + 1] - 3.0)
+    g[0, 0, 0] = 0.0
+    phi = torch.fft.irfftn(torch.fft.rfftn(rho) * g, s=(ng, ng, ng))
+    del rho, g
+    for dim in range(3):
+        want = 0.5 * (torch.roll(phi, 1, dim) - torch.roll(phi, -1, dim))
+        err = (torch.from_numpy(np.ascontiguousarray(f[dim])).cuda().reshape(ng, ng, ng) - want).abs().max()
+        assert float(err / want.abs().max()) < FIELD_RTOL
+    del phi, want, err
+    torch.cuda.empty_cache()
