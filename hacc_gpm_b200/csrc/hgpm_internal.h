@@ -73,6 +73,11 @@ cudaError_t launch_zy_fwd(int ng, unsigned long long* rho, float2* spec, int zs,
 cudaError_t launch_yz_inv_pair(int ng, float2* spec, float* out, int zs, const float2* tw, cudaStream_t s);
 cudaError_t launch_strided(int ng, bool inv, float2* data, int ncols, size_t rs, size_t ps, int nplanes, size_t cs,
                            int ncomp, const float2* tw, cudaStream_t s, const Slots& sl = Slots{}, int nslots = 1);
+// Density (left zeroed) to paired potential of a box of a side that
+// solve_small_supported names, in one kernel.
+bool solve_small_supported(int ng);
+cudaError_t launch_solve_small(int ng, unsigned long long* rho, float* out, double mean, const float2* tw,
+                               const double* cosq, double coeff, cudaStream_t s);
 // x pass fused with the Green's function: the potential's spectrum
 // G rho_k, transformed back along x, into out (one half-spectrum buffer).
 // (launch_xpotential_tma: the same pass fed by TMA, x pass choice 1.)

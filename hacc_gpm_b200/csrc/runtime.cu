@@ -757,16 +757,33 @@ static int forward_zy(hgpm_ctx* c) {
     return HGPM_OK;
 }
 
+// Whether the solve runs as one kernel: a side that fits, the kick gathers the
+// paired potential, and nothing asks for a pass of its own (a tuned y or x
+// pass, the plane kernels, or the clock of the phases).
+static bool solve_in_one_kernel(const hgpm_ctx* c) {
+    return solve_small_supported(c->ng) && kick_uses_phi2(c->kick_choice) && !c->tma && c->xmode != 1 && !c->plane &&
+           !c->timing;
+}
+
 extern "C" int hgpm_solve_gradient(hgpm_ctx* c) {
     if (!c) return HGPM_ERR_ARG;
     if (!c->rho_dirty) return fail(c, HGPM_ERR_STATE, "no deposited density (call hgpm_deposit first)");
     const int ng = c->ng, M = ng / 2;
+    const double coeff = 0.5 / ((double)ng * ng * ng);
+    if (solve_in_one_kernel(c)) {
+        PhaseScope ps(c, PH_POISSON);
+        CK(launch_solve_small(ng, c->rho64, c->force, mean_density(c), c->tw_ng, c->cosq, coeff, c->stream));
+        c->rho_dirty = false;
+        c->force_valid = c->phi_valid = false;
+        c->phi2_valid = true;
+        count(c, PH_POISSON, 1);
+        return HGPM_OK;
+    }
     int rc = forward_zy(c);
     if (rc) return rc;
     const size_t cs = (size_t)ng * ng * c->zs;
     {
         PhaseScope ps(c, PH_POISSON);
-        const double coeff = 0.5 / ((double)ng * ng * ng);
         if (c->xmode == 1)
             CK(launch_xpotential_tma(ng, c->spec, c->fspec, M + 1, c->zs, c->tw_ng, c->cosq, coeff, c->d_err + 1,
                                      c->stream));
@@ -823,11 +840,16 @@ static const float* ctx_phi(const hgpm_ctx* c) {
 extern "C" int hgpm_get_force(hgpm_ctx* c, float* f) {
     if (!c || !f) return HGPM_ERR_ARG;
     if (!c->force_valid && !c->phi_valid && c->phi2_valid) {
-        // the real potential from the potential's spectrum, which the solve
-        // leaves in place (the grid below overwrites the paired potential)
+        // the real potential (the grid below overwrites the paired one): from
+        // the potential's spectrum, which the solve leaves in place, or, where
+        // a solve may have formed none, the first halves of the paired records
         const int ng = c->ng;
-        CK(launch_zinv(ng, c->fspec, reinterpret_cast<float*>(c->fspec + (size_t)ng * ng * c->zs), ng * ng, c->zs,
-                       0, 0, 1, 1.0f, c->tw_ng, c->stream));
+        float2* phi = c->fspec + (size_t)ng * ng * c->zs;
+        if (solve_small_supported(ng))
+            CK(cudaMemcpy2DAsync(phi, 8, c->force, 16, 8, c->ncell / 2, cudaMemcpyDeviceToDevice, c->stream));
+        else
+            CK(launch_zinv(ng, c->fspec, reinterpret_cast<float*>(phi), ng * ng, c->zs, 0, 0, 1, 1.0f, c->tw_ng,
+                           c->stream));
         count(c, PH_ZINV, 1);
         c->phi_valid = true;
     }

@@ -547,3 +547,29 @@ def test_solve_of_large_sides_matches_double_fft(ng, np_side):
         assert float(err / want.abs().max()) < FIELD_RTOL
     del phi, want, err
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("ng,np_side", [(16, 16), (16, 32), (24, 24), (32, 32), (32, 16), (32, 64), (40, 40)])
+def test_one_kernel_solve_equals_passes(ng, np_side):
+    """The whole solve of a small box in one kernel and the separate passes
+    (which run while the phases are timed) leave the same bits: the state after
+    steps, the potential's force grid and an empty accumulator."""
+    x, v = lattice_state(np_side, ng, disp=1.5, vel=0.2, seed=11)
+    got = []
+    for timed in (False, True):
+        with make(ng, np_side) as s:
+            s.enable_timing(timed)
+            s.load_state(x, v)
+            s.cic()
+            s.solve_gradient()
+            first = s.get_force()
+            s.cic()
+            rho = s.get_density()
+            s.solve_gradient()
+            s.kick_drift(0.0123, 1.7, 0.3, 0.25, 2)
+            again = s.get_force()
+            xo, vo = s.store_state()
+        assert np.array_equal(first, again)
+        got.append((first, rho, xo, vo))
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
