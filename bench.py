@@ -138,9 +138,13 @@ def kernel_names(tuned, np_side, ng, plane=None):
             6: "zpass_c2r_kernel<NG> (the potential)"}.get(
         kick, "zpass_c2r_kernel<NG> (the potential) + gradient_kernel<8,3,2> (central differences, float4 force)")
     spill = "deposit_spill_kernel<%d,S,%d>" % (blk, 1024 if blk == 16 else 512)
+    # blocks that do not fit are queued for the spill pass, but by the 8^3
+    # column kernels and, in small boxes, the 16^3 one (they add them themselves)
+    direct, column = (9, ()) if blk == 16 else (5, (2, 4, 6, 7))
+    queues = dep != direct and (ng > 4 * np_side or not (dep in column or blk == 16 and dep == 8 and np_side <= 128))
     names = {
-        "deposit": DEPOSIT_NAMES[blk][dep] + ("" if dep == (9 if blk == 16 else 5) else " + %s (queued blocks)" % spill),
-        "fft_z_fwd": "zpass_r2c_kernel<NG,1>",
+        "deposit": DEPOSIT_NAMES[blk][dep] + (" + %s (queued blocks)" % spill if queues else ""),
+        "fft_z_fwd": "zpass_rho_kernel<NG>",
         "fft_y_fwd": "strided_tma_kernel<NG,0,0>" if ypass else "strided_kernel<NG,0>",
         "poisson_x": {1: "xpotential_tma_kernel<NG,256>"}.get(xpass, "xpot_kernel<NG>") +
                      " (forward x, Green's function, inverse x)",

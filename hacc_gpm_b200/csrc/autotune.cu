@@ -11,7 +11,7 @@
 //            the real potential (no force grid: the gradient kernel's time
 //            is charged to the others), CTA shape, units per CTA turn
 //            (launch_kick_drift candidates),
-//   y pass   TMA-fed persistent or plain strided transform,
+//   y pass   TMA-fed persistent or line-tile transform,
 //   x pass   TMA-fed persistent or line-tile fused Poisson transform.
 // hgpm_autotune times every candidate on the context's own current state
 // (CUDA events on its stream), keeps the default unless another candidate
@@ -241,8 +241,14 @@ extern "C" int hgpm_autotune(hgpm_ctx* c, int reps, int store, int choices[HGPM_
     c->tma = pick[HGPM_TUNE_YPASS] != 0;
     c->xmode = pick[HGPM_TUNE_XPASS];
     // a real force grid from the current positions for the kick candidates
+    // (deposited as for the kick that reads the window records, so that this
+    // candidate has them)
     c->rho_dirty = true;
+    const int kick0 = c->kick_choice;
+    for (int i = 0; i < kick_candidates(np, ng); ++i)
+        if (kick_reads_records(i)) c->kick_choice = i;
     int rc = hgpm_deposit(c);
+    c->kick_choice = kick0;
     if (rc) return rc;
     rc = hgpm_solve_gradient(c);
     if (rc) return rc;

@@ -431,10 +431,10 @@ extern "C" int hgpm_ens_release(hgpm_ensemble* E, int ci, int slot) {
     return HGPM_OK;
 }
 
-// Kernels of one class step: deposit (with its spill pass 2), z forward, y
+// Kernels of one class step: deposit (2 where it queues blocks), z forward, y
 // forward, x potential, y inverse, z inverse, (gradient,) kick, slot advance.
 static int step_kernels(const hgpm_ensemble* E, const EnsClass& k) {
-    return 6 + (kick_uses_phi(E->kick_choice) ? 0 : 1) + (deposit_records(E->dep_choice, k.np, k.ng, k.nslots) ? 2 : 1) +
+    return 6 + (kick_uses_phi(E->kick_choice) ? 0 : 1) + (deposit_queues(E->dep_choice, k.np, k.ng, k.nslots) ? 2 : 1) +
            kick_kernels(E->kick_choice, k.np, k.ng);
 }
 
@@ -466,7 +466,9 @@ static int class_step(hgpm_ensemble* E, EnsClass& k, cudaStream_t s) {
     p.vy = (float*)(b + 5 * a);
     p.vz = (float*)(b + 6 * a);
     const int* act = k.d_active;
-    ECK(launch_deposit(p, k.np, ng, mass, k.rho64, k.blkwin, k.dep_spill, s,
+    SpillList spill = k.dep_spill;
+    if (!kick_reads_records(E->kick_choice)) spill.over = nullptr;
+    ECK(launch_deposit(p, k.np, ng, mass, k.rho64, k.blkwin, spill, s,
                        Slots{act, k.part_stride, k.ncell, k.win_stride}, S, E->dep_choice));
     ECK(launch_zfwd_rho(ng, k.rho64, k.spec, k.zs, mean, k.tw_ng, s, Slots{act, k.ncell, k.spec_elems}, S));
     ECK(launch_strided(ng, false, k.spec, M + 1, (size_t)k.zs, (size_t)ng * k.zs, ng, 0, 1, k.tw_ng, s,

@@ -15,7 +15,7 @@ namespace hgpm {
 // A cluster of kPlaneCTAs CTAs works on one x plane at a time, planes
 // cid, cid + G, cid + 2G, ... (G clusters, as many as are resident at once).
 // Forward (zy_fwd_kernel): the R2C z pass of a plane's L-line tiles (int64
-// density in and zeroed, as zpass_r2c_kernel<NG,1>; every kPlaneCTAs-th tile
+// density in and zeroed, as zpass_rho_kernel<NG>; every kPlaneCTAs-th tile
 // per CTA), the cluster barrier (release / acquire at cluster scope) that
 // makes the plane's half spectrum visible to every CTA of the cluster, then
 // the y transform of the plane's PlaneCfg-column tiles in place.  The plane
@@ -49,7 +49,7 @@ __device__ __forceinline__ void plane_cluster_sync() {
 }
 
 // The R2C z pass of lines [line0, line0 + L) of the int64 density: the
-// arithmetic of zpass_r2c_kernel<NG, true>, the half spectrum written with
+// arithmetic of zpass_rho_kernel<NG>, the half spectrum written with
 // write-back stores.  Returns synchronised (the tile may be reused).
 template <int NG>
 __device__ __forceinline__ void zr2c_fix_tile(unsigned long long* __restrict__ in, float2* __restrict__ out, int line0,

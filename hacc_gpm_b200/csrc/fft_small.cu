@@ -143,8 +143,8 @@ __global__ void __cluster_dims__(SmallBox<NG>::CS, 1, 1) __launch_bounds__(Small
 }
 
 // The sides whose lines are two radices (one group of registers).  40 gains
-// least (36 against 39 us a step), so 64, the next such side, with twice the
-// cells for each of the 8 CTAs twice over, is left to the passes.
+// least (36 against 39 us a step), so 64, the next such side, with four times
+// its cells for each of the 8 CTAs, is left to the passes.
 bool solve_small_supported(int ng) { return ng == 16 || ng == 24 || ng == 32 || ng == 40; }
 
 cudaError_t launch_solve_small(int ng, unsigned long long* rho, float* out, double mean, const float2* tw,

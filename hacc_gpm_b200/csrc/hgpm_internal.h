@@ -129,6 +129,8 @@ int kick_kernels(int choice, int np_side, int ng);
 // Candidates that gather the real potential instead of the float4 force
 // grid (the step then skips gradient_kernel).
 bool kick_uses_phi(int choice);
+// The kick that reads the deposit's window records and its count of wide ones.
+bool kick_reads_records(int choice);
 // the kick gathers the paired potential (zpass_c2r with pair: cell z holds
 // (phi(z), phi(z+1)), 8 bytes per cell, in the force grid's space)
 bool kick_uses_phi2(int choice);
@@ -136,11 +138,12 @@ bool kick_uses_phi2(int choice);
 // default (used when the choice is -1).
 int deposit_candidates(int np_side, int ng);
 int deposit_default(int np_side, int ng, int nslots = 1);
-// Whether candidate `choice` writes the blocks' window records and launches a
-// spill pass (all but the direct one).
+// Whether candidate `choice` writes the blocks' window records (all but the
+// direct one).
 bool deposit_records(int choice, int np_side, int ng, int nslots = 1);
-// Built-in kick candidate (without tuning): the paired potential for 16^3
-// blocks, the real potential for 8^3 blocks.
+// Whether it queues blocks for a spill pass (a second kernel).
+bool deposit_queues(int choice, int np_side, int ng, int nslots = 1);
+// Built-in kick candidate (without tuning): the paired potential.
 int kick_default(int np_side, int ng);
 // Blocks too wide for a kernel's window are queued in `spill` (the deposit's
 // and the kick's own lists) and run one particle per thread after the

@@ -36,7 +36,6 @@ __device__ __forceinline__ float green(double s, double coeff) {
 }
 
 struct PotentialOp {
-    static constexpr int kOut = 1;
     const double* cosq;  // cos(k_i) - 1, one entry per grid index
     double coeff;        // 0.5 / ng^3
     __device__ __forceinline__ float2 pre(int ix, int iy, int iz, float2 v) const {
@@ -50,7 +49,6 @@ struct PotentialOp {
         // operator between its transforms gets the same bits
         return make_float2(__fmul_rn(v.x, g), __fmul_rn(v.y, g));
     }
-    __device__ __forceinline__ float2 comp(int, int, int, int, float2 t) const { return t; }
 };
 
 // Zel'dovich displacement (initializer.cpp:10-117): ScaleAmplitudes by
@@ -58,7 +56,6 @@ struct PotentialOp {
 // then transformDensityField (transform_density_field_initializer.cu:72-112):
 // s_d = (Im k_d, -Re k_d) / (k^2 delta).
 struct ICOp {
-    static constexpr int kOut = 3;  // the x pass stores all three components
     const double* table;
     int nbins;
     double k_delta;

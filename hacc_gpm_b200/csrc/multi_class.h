@@ -9,9 +9,9 @@
 // finds its unit's class in the table below and runs that class's code for
 // that unit: the same device bodies the single-class kernels run
 // (bit-identical results), the FFT ones dispatched on the class's grid side.
-// The deposit and the kick are persistent grids walking the units; the FFT
-// passes launch one CTA per unit.  Per step: a counter reset, the deposit,
-// its spill pass, the five FFT passes (z, y, x with the Green's function, y,
+// The kick is a persistent grid walking the units; the other passes launch one
+// CTA per unit.  Per step: a counter reset, the deposit, the pass over the
+// parts of blocks it left over, the five FFT passes (z, y, x with the Green's function, y,
 // and z to the paired potential), the kick gathering the paired potential
 // with both drifts, and the slot advance: ten launches whatever the number of
 // classes.

@@ -605,13 +605,37 @@ __global__ void __launch_bounds__(NT, MINB) deposit_w32_kernel(ParticleSoA p, in
     }
 }
 
+// The 8 fixed-point corner weights of one particle added straight to the
+// int64 grid (blocks too wide for a shared-memory window).
+template <bool SMALL>
+__device__ __forceinline__ void deposit_global(unsigned long long* __restrict__ rho, uint32_t c, float dx, float dy,
+                                               float dz, float mass, int ng) {
+    unsigned long long q[8];
+    cic_fixed<SMALL>(dx, dy, dz, mass, q);
+    const int ix = cell_x(c), iy = cell_y(c), iz = cell_z(c);
+    const int ix1 = ix + 1 == ng ? 0 : ix + 1;
+    const int iy1 = iy + 1 == ng ? 0 : iy + 1;
+    const int iz1 = iz + 1 == ng ? 0 : iz + 1;
+    const size_t sx[2] = {(size_t)ix * ng * ng, (size_t)ix1 * ng * ng};
+    const size_t sy[2] = {(size_t)iy * ng, (size_t)iy1 * ng};
+    const size_t sz[2] = {(size_t)iz, (size_t)iz1};
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc) atomicAdd(&rho[sx[a] + sy[b] + sz[cc]], q[(a * 2 + b) * 2 + cc]);
+}
+
 // Column deposit: 32-bit windows (as deposit_w32_kernel) with one thread per
 // (y, z) column of the block, which walks the column's B particles along x
 // with the next PF in flight in a register ring.  A block whose window is
 // wider than the cap but whose two x-halves (x < B/2, x >= B/2) each fit is
 // deposited as two halves, one after the other, each with its own window,
-// wrap check and flush; only blocks whose halves do not fit either (or that
-// wrap) go to deposit_spill_kernel.
+// wrap check and flush.  Blocks whose halves do not fit either (or that wrap):
+// QUEUE leaves them to deposit_spill_kernel, else their particles are added
+// straight to the int64 grid, in the same CTA, beside other blocks' windows
+// (see deposit_default_choice).
 // Adds the column range [k0, k0 + len) into the window.  RET: each atomic
 // returns the cell's old value, and *wrapped records whether any old value
 // had its top bit set: an add of v < 2^30 (mass <= 64) can wrap only a cell
@@ -787,10 +811,11 @@ __device__ __forceinline__ bool column_pass(const ParticleSoA& p, int i0, int k0
     return tot == 0;
 }
 
-// Block blk of one box: p, rho, recs (window records, may be null), the
-// box's spill queue (items, cnt) and wide-window counter (over, may be
-// null).  The single-class kernel below and the multi-class deposit run it.
-template <int B, int PF, int CHK, bool CHAIN = false>
+// Block blk of one box: p, rho, recs (window records, may be null) and the
+// box's wide-window counter (over, may be null).  The single-class kernel below
+// and the multi-class deposit run it.  QUEUE: the left-over parts go to the
+// box's spill queue (items, cnt) instead of the grid.
+template <int B, int PF, int CHK, bool CHAIN, bool QUEUE>
 __device__ __forceinline__ void deposit_col_body(ParticleSoA p, int np_side, int ng, float mass,
                                                  unsigned long long* __restrict__ rho, int cap_cells,
                                                  int* __restrict__ recs, int* __restrict__ items, int* cnt,
@@ -858,59 +883,47 @@ __device__ __forceinline__ void deposit_col_body(ParticleSoA p, int np_side, int
     const long long vol = (long long)wx * wy * wz;
     if (tid == 0 && over && vol > kWin4Cap) atomicAdd(over, 1);
     unsigned* w0 = reinterpret_cast<unsigned*>(win);
-    // queued part: 0 the whole block, 2 its upper x-half (the lower half
-    // flushed); at most one item per block
-    int queue = -1;
+    // particles of each column left to add straight, from x = rest on: the
+    // whole block, or its upper x-half (the lower half flushed)
+    int rest = B;
     if (vol <= cap_cells) {
-        if (!column_pass<B, PF, CHK, CHAIN>(p, tid, 0, B, mass, w0, wsum, bb, ox, oy, oz, ng, rho)) queue = 0;
+        if (!column_pass<B, PF, CHK, CHAIN>(p, tid, 0, B, mass, w0, wsum, bb, ox, oy, oz, ng, rho)) rest = 0;
     } else {
         auto hvol = [&](int h) {
             const int* q = bb + 6 + 6 * h;
             return (long long)(q[3] - q[0] + 2) * (q[4] - q[1] + 2) * (q[5] - q[2] + 2);
         };
         if (hvol(0) <= cap_cells && hvol(1) <= cap_cells) {
-            if (!column_pass<B, PF, CHK, CHAIN>(p, tid, 0, B / 2, mass, w0, wsum, bb + 6, ox, oy, oz, ng, rho)) queue = 0;
+            if (!column_pass<B, PF, CHK, CHAIN>(p, tid, 0, B / 2, mass, w0, wsum, bb + 6, ox, oy, oz, ng, rho)) rest = 0;
             else if (!column_pass<B, PF, CHK, CHAIN>(p, tid, B / 2, B / 2, mass, w0, wsum, bb + 12, ox, oy, oz, ng, rho))
-                queue = 2;
+                rest = B / 2;
         } else {
-            queue = 0;
+            rest = 0;
         }
     }
-    if (queue >= 0 && tid == 0) items[atomicAdd(cnt, 1)] = blk * 4 + queue;
+    if (QUEUE) {
+        if (rest < B && tid == 0) items[atomicAdd(cnt, 1)] = blk * 4 + (rest ? 2 : 0);
+        return;
+    }
+    // (32-bit windows: mass <= 64, so every weight fits 32 bits)
+#pragma unroll 1
+    for (int k = rest; k < B; ++k) {
+        const int i = tid + k * NT;
+        deposit_global<true>(rho, __ldg(&p.cell[i]), __ldg(&p.ox[i]), __ldg(&p.oy[i]), __ldg(&p.oz[i]), mass, ng);
+    }
 }
 
-template <int B, int MINB, int PF, int CHK = 0, bool CHAIN = false>
+template <int B, int MINB, int PF, int CHK = 0, bool CHAIN = false, bool QUEUE = (B == 16)>
 __global__ void __launch_bounds__(B * B, MINB) deposit_col_kernel(ParticleSoA p, int np_side, int ng, float mass,
                                                                   unsigned long long* __restrict__ rho, int cap_cells,
                                                                   int* __restrict__ blkwin, SpillList spill, Slots sl) {
     const int slot = blockIdx.y;
     if (slot_idle(sl, slot)) return;
-    deposit_col_body<B, PF, CHK, CHAIN>(offset_soa(p, (size_t)slot * sl.s0), np_side, ng, mass, rho + (size_t)slot * sl.s1,
-                                 cap_cells, blkwin ? blkwin + (size_t)slot * sl.s2 : nullptr,
-                                 spill.items + (size_t)slot * spill.nblocks, spill.cnt + slot,
-                                 spill.over ? spill.over + slot : nullptr, blockIdx.x);
-}
-
-// The 8 fixed-point corner weights of one particle added straight to the
-// int64 grid (blocks too wide for a shared-memory window).
-template <bool SMALL>
-__device__ __forceinline__ void deposit_global(unsigned long long* __restrict__ rho, uint32_t c, float dx, float dy,
-                                               float dz, float mass, int ng) {
-    unsigned long long q[8];
-    cic_fixed<SMALL>(dx, dy, dz, mass, q);
-    const int ix = cell_x(c), iy = cell_y(c), iz = cell_z(c);
-    const int ix1 = ix + 1 == ng ? 0 : ix + 1;
-    const int iy1 = iy + 1 == ng ? 0 : iy + 1;
-    const int iz1 = iz + 1 == ng ? 0 : iz + 1;
-    const size_t sx[2] = {(size_t)ix * ng * ng, (size_t)ix1 * ng * ng};
-    const size_t sy[2] = {(size_t)iy * ng, (size_t)iy1 * ng};
-    const size_t sz[2] = {(size_t)iz, (size_t)iz1};
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b)
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc) atomicAdd(&rho[sx[a] + sy[b] + sz[cc]], q[(a * 2 + b) * 2 + cc]);
+    deposit_col_body<B, PF, CHK, CHAIN, QUEUE>(offset_soa(p, (size_t)slot * sl.s0), np_side, ng, mass,
+                                               rho + (size_t)slot * sl.s1, cap_cells,
+                                               blkwin ? blkwin + (size_t)slot * sl.s2 : nullptr,
+                                               spill.items + (size_t)slot * spill.nblocks, spill.cnt + slot,
+                                               spill.over ? spill.over + slot : nullptr, blockIdx.x);
 }
 
 // Direct deposit: a thread per particle adds its 8 fixed-point weights
@@ -1799,6 +1812,7 @@ using DepositFn = void (*)(ParticleSoA, int, int, float, unsigned long long*, in
 struct DepositCfg {
     DepositFn fn;
     int nt, cap, cell_bytes;
+    bool queues;  // leaves blocks to deposit_spill_kernel (not the 8^3 column kernels)
 };
 
 constexpr int kDepositCands = 12;
@@ -1824,38 +1838,38 @@ template <int B, bool SMALL>
 static int deposit_candidates(int cap_default, bool w32, DepositCfg* out) {
     int n = 0;
     if constexpr (B == 16) {
-        out[n++] = {deposit_tiled_kernel<B, SMALL, 256, 3>, 256, cap_default, 8};
-        out[n++] = {deposit_tiled_kernel<B, SMALL, 512, 2>, 512, 13824, 8};
-        out[n++] = {deposit_tiled_kernel<B, SMALL, 1024, 1>, 1024, kBigCap, 8};
+        out[n++] = {deposit_tiled_kernel<B, SMALL, 256, 3>, 256, cap_default, 8, true};
+        out[n++] = {deposit_tiled_kernel<B, SMALL, 512, 2>, 512, 13824, 8, true};
+        out[n++] = {deposit_tiled_kernel<B, SMALL, 1024, 1>, 1024, kBigCap, 8, true};
         if (w32) {
-            out[n++] = {deposit_w32_kernel<B, 512, 2, true>, 512, 13824, 4};
-            out[n++] = {deposit_w32_kernel<B, 256, 4, true, 4>, 256, 13312, 4};
-            out[n++] = {deposit_col_kernel<B, 4, 4>, 256, 13312, 4};
-            out[n++] = {deposit_col_kernel<B, 4, 2>, 256, 13312, 4};
-            out[n++] = {deposit_col_kernel<B, 3, 4>, 256, 18432, 4};
-            out[n++] = {deposit_col_kernel<B, 4, 4, 1>, 256, 13312, 4};
+            out[n++] = {deposit_w32_kernel<B, 512, 2, true>, 512, 13824, 4, true};
+            out[n++] = {deposit_w32_kernel<B, 256, 4, true, 4>, 256, 13312, 4, true};
+            out[n++] = {deposit_col_kernel<B, 4, 4>, 256, 13312, 4, true};
+            out[n++] = {deposit_col_kernel<B, 4, 2>, 256, 13312, 4, true};
+            out[n++] = {deposit_col_kernel<B, 3, 4>, 256, 18432, 4, true};
+            out[n++] = {deposit_col_kernel<B, 4, 4, 1>, 256, 13312, 4, true};
         } else {
             // the split window with the same threads per CTA
             const int same_nt[6] = {1, 0, 0, 0, 0, 0};
             for (int i = 0; i < 6; ++i) out[n + i] = out[same_nt[i]];
             n += 6;
         }
-        out[n++] = {nullptr, 0, 0, 0};
-        out[n++] = w32 ? DepositCfg{deposit_col_kernel<B, 4, 4, 2>, 256, 13312, 4} : out[0];
-        out[n++] = w32 ? DepositCfg{deposit_col_kernel<B, 4, 4, 1, true>, 256, 13312, 4} : out[0];
+        out[n++] = {nullptr, 0, 0, 0, false};
+        out[n++] = w32 ? DepositCfg{deposit_col_kernel<B, 4, 4, 2>, 256, 13312, 4, true} : out[0];
+        out[n++] = w32 ? DepositCfg{deposit_col_kernel<B, 4, 4, 1, true>, 256, 13312, 4, true} : out[0];
     } else {
-        out[n++] = {deposit_tiled_kernel<B, SMALL, 256, 3>, 256, cap_default, 8};
+        out[n++] = {deposit_tiled_kernel<B, SMALL, 256, 3>, 256, cap_default, 8, true};
         if (w32) {
-            out[n++] = {deposit_w32_kernel<B, 256, 4, true, 2>, 256, 13312, 4};
-            out[n++] = {deposit_col_kernel<B, 12, 4>, B * B, 4096, 4};
-            out[n++] = {deposit_w32_kernel<B, 512, 2, true, 1>, 512, kBigCap, 4};
-            out[n++] = {deposit_col_kernel<B, 12, 4, 1>, B * B, 4096, 4};
+            out[n++] = {deposit_w32_kernel<B, 256, 4, true, 2>, 256, 13312, 4, true};
+            out[n++] = {deposit_col_kernel<B, 12, 4>, B * B, 4096, 4, false};
+            out[n++] = {deposit_w32_kernel<B, 512, 2, true, 1>, 512, kBigCap, 4, true};
+            out[n++] = {deposit_col_kernel<B, 12, 4, 1>, B * B, 4096, 4, false};
         } else {
             for (int i = 0; i < 4; ++i) out[n++] = out[0];
         }
-        out[n++] = {nullptr, 0, 0, 0};
-        out[n++] = w32 ? DepositCfg{deposit_col_kernel<B, 12, 4, 2>, B * B, 4096, 4} : out[0];
-        out[n++] = w32 ? DepositCfg{deposit_col_kernel<B, 12, 4, 1, true>, B * B, 4096, 4} : out[0];
+        out[n++] = {nullptr, 0, 0, 0, false};
+        out[n++] = w32 ? DepositCfg{deposit_col_kernel<B, 12, 4, 2>, B * B, 4096, 4, false} : out[0];
+        out[n++] = w32 ? DepositCfg{deposit_col_kernel<B, 12, 4, 1, true>, B * B, 4096, 4, false} : out[0];
     }
     return n;
 }
@@ -1874,6 +1888,18 @@ static int deposit_candidates(int cap_default, bool w32, DepositCfg* out) {
 // the other windows), otherwise the column kernel (returned-value wraps 103.6
 // us at 200^3, window-sum check 106.7).  A batched launch has the blocks of
 // all its slots.
+//   Blocks left over by the column kernels (too wide, or wrapped): the spill
+// pass and its counters cost every step three launches (8 us); adding the
+// particles straight to the grid costs the deposit itself most where there are
+// many such blocks.  us a deposit mid-run, straight / spill pass: 8^3 blocks
+// 27 / 35 at 120^3, 95 / 103 at 200^3 (a clustered step, 100 steps on: 132 /
+// 161 and 462 / 580); 16^3 blocks 33 / 40 at 128^3, 150 / 152 at 256^3 (a
+// clustered step 948 / 916), 1085 / 1062 at 512^3.  So 8^3 blocks add
+// straight, and 16^3 blocks up to 512 of them.
+static bool deposit_straight(int choice, int np_side, int nslots) {
+    return choice == 8 && (long long)(np_side / 16) * (np_side / 16) * (np_side / 16) * nslots <= 512;
+}
+
 template <int B>
 static int deposit_default_choice(int np_side, int ng, int nslots) {
     const long long blocks = (long long)(np_side / B) * (np_side / B) * (np_side / B) * nslots;
@@ -1889,7 +1915,11 @@ static cudaError_t deposit_impl(const ParticleSoA& p, int np_side, int ng, float
     DepositCfg cands[kDepositCands];
     const int ncand = deposit_candidates<B, SMALL>(cap, mass <= 64.0f, cands);
     const int mode = choice >= 0 && choice < ncand ? choice : deposit_default_choice<B>(np_side, ng, nslots);
-    const DepositCfg& cfg = cands[mode];
+    DepositCfg cfg = cands[mode];
+    if (deposit_straight(mode, np_side, nslots)) {
+        if constexpr (B == 16)
+            if (mass <= 64.0f) cfg.fn = deposit_col_kernel<B, 4, 4, 1, false, false>, cfg.queues = false;
+    }
     const DepositFn k = cfg.fn;
     if (!k) {  // direct: n <= 1024^3
         const int n = np_side * np_side * np_side;
@@ -1901,13 +1931,13 @@ static cudaError_t deposit_impl(const ParticleSoA& p, int np_side, int ng, float
     const int smem = cap * cfg.cell_bytes;
     cudaError_t e = smem_attr_once((const void*)k, smem, nt);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(spill.cnt, 0, sizeof(int) * nslots, s);
+    if (cfg.queues) e = cudaMemsetAsync(spill.cnt, 0, sizeof(int) * nslots, s);
     if (e == cudaSuccess && spill.over) e = cudaMemsetAsync(spill.over, 0, sizeof(int) * nslots, s);
     if (e != cudaSuccess) return e;
     const int nb = np_side / B;
     k<<<dim3(nb * nb * nb, nslots), nt, smem, s>>>(p, np_side, ng, mass, rho, cap, blkwin, spill, sl);
     e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || !cfg.queues) return e;
     constexpr int NTS = B * B * B >= 1024 ? 1024 : B * B * B;
     auto ks = deposit_spill_kernel<B, SMALL, NTS>;
     e = smem_attr_once((const void*)ks, kBigCap * 8, NTS);
@@ -1915,6 +1945,13 @@ static cudaError_t deposit_impl(const ParticleSoA& p, int np_side, int ng, float
     const int per_slot = num_sms() / nslots > 1 ? num_sms() / nslots : 1;  // about one CTA per SM in all
     ks<<<dim3(per_slot, nslots), NTS, kBigCap * 8, s>>>(p, np_side, ng, mass, rho, blkwin, spill, sl);
     return cudaGetLastError();
+}
+
+bool deposit_queues(int choice, int np_side, int ng, int nslots) {
+    if (choice < 0 || choice >= deposit_candidates(np_side, ng)) choice = deposit_default(np_side, ng, nslots);
+    if (ng > 4 * np_side) return deposit_records(choice, np_side, ng, nslots);  // no 32-bit windows
+    if (block_side(np_side, ng) == 16) return choice != 9 && !deposit_straight(choice, np_side, nslots);
+    return choice < 2 || choice == 3;
 }
 
 bool deposit_records(int choice, int np_side, int ng, int nslots) {
@@ -1965,6 +2002,7 @@ int kick_candidates(int np_side, int ng) {
     return kKickCands;
 }
 
+bool kick_reads_records(int choice) { return choice == kKickWindowed; }
 bool kick_uses_phi(int choice) { return choice >= kKickPhiFirst && choice < kKickCands; }
 bool kick_uses_phi2(int choice) { return choice == kKickPhi2; }
 
@@ -2210,24 +2248,32 @@ __global__ void __launch_bounds__(256, 4) mc_deposit_kernel(const __grid_constan
             deposit_global<true>(rho, __ldg(&p.cell[i]), __ldg(&p.ox[i]), __ldg(&p.oy[i]), __ldg(&p.oz[i]), c.mass, c.ng);
         return;
     }
-    deposit_col_body<16, 4, 1>(offset_soa(c.p, (size_t)slot * c.part_stride), c.np, c.ng, c.mass,
-                               c.rho64 + (size_t)slot * c.ncell, kMCDepCap, c.blkwin + (size_t)slot * c.win_stride,
-                               c.spill.items + (size_t)slot * c.spill.nblocks, c.spill.cnt + slot,
-                               c.spill.over ? c.spill.over + slot : nullptr, blk);
+    deposit_col_body<16, 4, 1, false, true>(offset_soa(c.p, (size_t)slot * c.part_stride), c.np, c.ng, c.mass,
+                                            c.rho64 + (size_t)slot * c.ncell, kMCDepCap,
+                                            c.blkwin + (size_t)slot * c.win_stride,
+                                            c.spill.items + (size_t)slot * c.spill.nblocks, c.spill.cnt + slot,
+                                            c.spill.over ? c.spill.over + slot : nullptr, blk);
 }
 
-// deposit_spill_kernel over every slot's queue: blockIdx.y = global slot
-__global__ void __launch_bounds__(1024, 1) mc_spill_kernel(const __grid_constant__ MCTable t) {
+// Every slot's queue of left-over parts, added straight to the grid, an x-plane
+// of a block (256 particles) to a CTA at a time: blockIdx.y = global slot.  (One
+// 1024-thread CTA to a block with a window of its own, as deposit_spill_kernel,
+// took 14.6 us a step for the few blocks there are.)
+__global__ void __launch_bounds__(256) mc_spill_kernel(const __grid_constant__ MCTable t) {
     int k = 0, slot = blockIdx.y;
     while (k < t.n && slot >= t.c[k].nslots) slot -= t.c[k++].nslots;
     if (k >= t.n) return;
     const MCClass& c = t.c[k];
     if (c.active && !c.active[slot]) return;
-    const int cnt = c.spill.cnt[slot];
-    if ((int)blockIdx.x >= cnt) return;
-    deposit_spill_body<16, true, 1024>(offset_soa(c.p, (size_t)slot * c.part_stride), c.np, c.ng, c.mass,
-                                       c.rho64 + (size_t)slot * c.ncell, c.blkwin + (size_t)slot * c.win_stride,
-                                       c.spill.items + (size_t)slot * c.spill.nblocks, cnt, blockIdx.x, gridDim.x);
+    const int planes = c.spill.cnt[slot] * 16;
+    const ParticleSoA p = offset_soa(c.p, (size_t)slot * c.part_stride);
+    unsigned long long* rho = c.rho64 + (size_t)slot * c.ncell;
+    for (int u = blockIdx.x; u < planes; u += gridDim.x) {
+        const int item = c.spill.items[(size_t)slot * c.spill.nblocks + u / 16], x = u % 16;
+        if ((item & 2) && x < 8) continue;  // the lower half is in the grid
+        const size_t i = (size_t)(item / 4) * 4096 + x * 256 + threadIdx.x;
+        deposit_global<true>(rho, __ldg(&p.cell[i]), __ldg(&p.ox[i]), __ldg(&p.oy[i]), __ldg(&p.oz[i]), c.mass, c.ng);
+    }
 }
 
 // kick_phi_kernel's arithmetic (the paired potential) over units of 1024
@@ -2263,15 +2309,14 @@ __global__ void __launch_bounds__(1024, 1) mc_kick_kernel(const __grid_constant_
     }
 }
 
+// a CTA per class (7 us a step for five classes one after the other)
 __global__ void mc_advance_kernel(const __grid_constant__ MCTable t) {
-    for (int k = 0; k < t.n; ++k) {
-        const MCClass& c = t.c[k];
-        for (int i = threadIdx.x; i < c.nslots; i += blockDim.x) {
-            if (!c.active[i]) continue;
-            const int st = c.step[i] + 1;
-            c.step[i] = st;
-            if (st >= c.nsteps[i]) c.active[i] = 0;
-        }
+    const MCClass& c = t.c[blockIdx.x];
+    for (int i = threadIdx.x; i < c.nslots; i += blockDim.x) {
+        if (!c.active[i]) continue;
+        const int st = c.step[i] + 1;
+        c.step[i] = st;
+        if (st >= c.nsteps[i]) c.active[i] = 0;
     }
 }
 
@@ -2321,11 +2366,8 @@ cudaError_t mc_step(const MCTable& base, cudaStream_t s) {
         if (e != cudaSuccess) return e;
     }
     {
-        const int per = num_sms() / nslots > 1 ? num_sms() / nslots : 1;
-        auto ks = mc_spill_kernel;
-        e = smem_attr_once((const void*)ks, kBigCap * 8, 1024);
-        if (e != cudaSuccess) return e;
-        ks<<<dim3(per, nslots), 1024, kBigCap * 8, s>>>(base);
+        const int per = 6 * num_sms() / nslots > 1 ? 6 * num_sms() / nslots : 1;
+        mc_spill_kernel<<<dim3(per, nslots), 256, 0, s>>>(base);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -2337,7 +2379,7 @@ cudaError_t mc_step(const MCTable& base, cudaStream_t s) {
     for (int k = 0; k < base.n; ++k) tk.u0[k + 1] = tk.u0[k] + base.c[k].nblocks * 4 * base.c[k].nslots;
     e = mc_persistent((const void*)mc_kick_kernel, tk, 1024, 0, s);
     if (e != cudaSuccess) return e;
-    return cudaLaunchKernel((const void*)mc_advance_kernel, dim3(1), dim3(256), pargs, 0, s);
+    return cudaLaunchKernel((const void*)mc_advance_kernel, dim3(base.n), dim3(128), pargs, 0, s);
 }
 
 }  // namespace hgpm

@@ -703,10 +703,12 @@ static double mean_density(const hgpm_ctx* c) {
 
 static int deposit_impl(hgpm_ctx* c) {
     if (c->rho_dirty) CK(cudaMemsetAsync(c->rho64, 0, c->ncell * 8, c->stream));
-    CK(launch_deposit(c->part, c->np, c->ng, cic_mass(c->ng, c->np), c->rho64, c->blkwin, c->dep_spill, c->stream,
+    SpillList spill = c->dep_spill;
+    if (!kick_reads_records(c->kick_choice)) spill.over = nullptr;
+    CK(launch_deposit(c->part, c->np, c->ng, cic_mass(c->ng, c->np), c->rho64, c->blkwin, spill, c->stream,
                       Slots{}, 1, c->dep_choice));
-    c->win_valid = deposit_records(c->dep_choice, c->np, c->ng);
-    count(c, PH_DEPOSIT, c->win_valid ? 2 : 1);  // windowed pass + spill pass, or the direct one
+    c->win_valid = kick_reads_records(c->kick_choice) && deposit_records(c->dep_choice, c->np, c->ng);
+    count(c, PH_DEPOSIT, deposit_queues(c->dep_choice, c->np, c->ng) ? 2 : 1);
     c->rho_dirty = true;
     return HGPM_OK;
 }

@@ -549,6 +549,38 @@ def test_solve_of_large_sides_matches_double_fft(ng, np_side):
     torch.cuda.empty_cache()
 
 
+@pytest.mark.parametrize("ng,np_side,choice", [(32, 32, "9"), (32, 32, "8"), (64, 64, "8"), (40, 40, "4"), (64, 32, "1"),
+                                               (64, 32, "0"), (128, 16, "0"), (48, 96, None)])
+def test_dense_cells_reach_the_solve(ng, np_side, choice, monkeypatch):
+    """Half the particles in a few cells, far from their blocks' windows and
+    thousands of units of weight in each: the forces match the oracle's on the
+    exact density, and the next deposits start from a clean accumulator."""
+    if choice is None:
+        monkeypatch.delenv("HGPM_DEPOSIT", raising=False)
+    else:
+        monkeypatch.setenv("HGPM_DEPOSIT", choice)
+    x, v = lattice_state(np_side, ng, disp=1.0, vel=0.0, seed=3)
+    hot = x.copy()
+    for k, at in enumerate(((1.5, 2.0, ng - 0.5), (0.0, 0.0, 0.0), (ng - 1.0, 3.25, 7.0), (5.0, 5.0, 5.0))):
+        hot[k * 2::8] = at
+    with make(ng, np_side) as s:
+        s.load_state(hot, v)
+        s.cic()
+        rho = s.get_density()
+        s.solve_gradient()
+        f = s.get_force()
+        s.load_state(x, v)
+        s.cic()
+        clean = s.get_density()
+        s.cic()
+        again = s.get_density()
+    ro = O.cic_deposit(hot.astype(np.float64), ng, O.cic_mass(ng, np_side))
+    assert rho.max() > 512 and np.abs(rho - ro).max() <= 1e-6 * ro.max()
+    assert rel_max_err(f, O.solve_gradient(rho.astype(np.float64), ref_quirks=True)) < FIELD_RTOL
+    rc = O.cic_deposit(x.astype(np.float64), ng, O.cic_mass(ng, np_side))
+    assert np.abs(clean - rc).max() <= 1e-6 * rc.max() and np.array_equal(clean, again)
+
+
 @pytest.mark.parametrize("ng,np_side", [(16, 16), (16, 32), (24, 24), (32, 32), (32, 16), (32, 64), (40, 40)])
 def test_one_kernel_solve_equals_passes(ng, np_side):
     """The whole solve of a small box in one kernel and the separate passes
