@@ -19,6 +19,8 @@ struct PhaseRec {
     cudaEvent_t a, b;
 };
 
+constexpr size_t kPinChunks = 4, kPinChunk = 512 << 10;  // copy_out's ring
+
 struct hgpm_ctx {
     hgpm_params p;
     int device = 0;
@@ -64,6 +66,8 @@ struct hgpm_ctx {
     int dep_choice = -1;
     int kick_choice = 0;
     float* stage = nullptr;     // AoS float3 x, v staging (lazy)
+    cudaEvent_t pin_ready[kPinChunks] = {};  // copy_out's chunks (lazy)
+    bool pins = false;          // counted among the users of the page-locked rings
     double* pk_part = nullptr;  // P(k) partial sums (lazy)
     unsigned long long* pk_pcnt = nullptr;
     double* pk_sum = nullptr;

@@ -476,6 +476,8 @@ int ctx_set_rl_tables(hgpm_ctx* c) {
     return HGPM_OK;
 }
 
+static void pin_leave();  // the page-locked rings of copy_out
+
 extern "C" void hgpm_destroy(hgpm_ctx* c) {
     if (!c) return;
     if (c->stream) cudaStreamSynchronize(c->stream);
@@ -495,6 +497,9 @@ extern "C" void hgpm_destroy(hgpm_ctx* c) {
         cudaEventDestroy(r.b);
     }
     for (auto e : c->free_events) cudaEventDestroy(e);
+    for (auto e : c->pin_ready)
+        if (e) cudaEventDestroy(e);
+    if (c->pins) pin_leave();
     if (c->stream && !c->view) cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -535,6 +540,108 @@ static int ensure_stage(hgpm_ctx* c) {
     return HGPM_OK;
 }
 
+// Page-locked rings for copy_out, shared by the contexts: a ring costs 3 ms to
+// allocate, so a context takes one for the length of a copy.  At most
+// kPinKeep are kept between copies, and none once the last context that
+// copied is gone.
+namespace {
+constexpr int kPinKeep = 4;
+std::mutex pin_mutex;
+char* pin_free[kPinKeep];
+int pin_nfree = 0, pin_users = 0;
+
+struct PinRing {
+    char* p = nullptr;
+    explicit PinRing(bool want) {
+        if (!want) return;
+        {
+            std::lock_guard<std::mutex> g(pin_mutex);
+            if (pin_nfree > 0) {
+                p = pin_free[--pin_nfree];
+                return;
+            }
+        }
+        if (cudaHostAlloc((void**)&p, kPinChunks * kPinChunk, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+    }
+    ~PinRing() {
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> g(pin_mutex);
+            if (pin_nfree < kPinKeep) {
+                pin_free[pin_nfree++] = p;
+                return;
+            }
+        }
+        cudaFreeHost(p);
+    }
+};
+}  // namespace
+
+static void pin_join() {
+    std::lock_guard<std::mutex> g(pin_mutex);
+    ++pin_users;
+}
+
+static void pin_leave() {
+    char* drop[kPinKeep];
+    int n = 0;
+    {
+        std::lock_guard<std::mutex> g(pin_mutex);
+        if (--pin_users == 0)
+            while (pin_nfree > 0) drop[n++] = pin_free[--pin_nfree];
+    }
+    while (n > 0) cudaFreeHost(drop[--n]);
+}
+
+// The staged state to the caller's arrays.  Into pageable memory the driver
+// copies 6.3 MB (64^3) in 1.02 ms; through a ring of page-locked chunks, the
+// next ones on their way while the host copies one out, it is the host's copy
+// alone (0.35 ms; five steps of 64^3 between host arrays 2.41 -> 1.70 ms).
+// Page-locked (or device) destinations are copied directly.
+static int copy_out(hgpm_ctx* c, float* x, float* v) {
+    const size_t bytes = c->npart * 3 * sizeof(float);
+    char* dst[2] = {(char*)x, (char*)v};
+    const char* src[2] = {(const char*)c->stage, (const char*)(c->stage + 3 * c->npart)};
+    bool pageable = bytes >= kPinChunk;  // below it the driver's copy is as fast
+    for (int a = 0; a < 2 && pageable; ++a) {
+        cudaPointerAttributes at;
+        CK(cudaPointerGetAttributes(&at, dst[a]));
+        pageable = at.type == cudaMemoryTypeUnregistered;
+    }
+    if (pageable && !c->pins) {
+        for (auto& e : c->pin_ready)
+            if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        pin_join();
+        c->pins = true;
+    }
+    PinRing ring(pageable);
+    if (!ring.p) {
+        for (int a = 0; a < 2; ++a) CK(cudaMemcpyAsync(dst[a], src[a], bytes, cudaMemcpyDeviceToHost, c->stream));
+        return HGPM_OK;
+    }
+    const size_t per = (bytes + kPinChunk - 1) / kPinChunk, n = 2 * per;
+    auto len = [&](size_t i) { return std::min(kPinChunk, bytes - i % per * kPinChunk); };
+    auto fetch = [&](size_t i) {
+        cudaError_t e = cudaMemcpyAsync(ring.p + i % kPinChunks * kPinChunk, src[i / per] + i % per * kPinChunk, len(i),
+                                        cudaMemcpyDeviceToHost, c->stream);
+        return e != cudaSuccess ? e : cudaEventRecord(c->pin_ready[i % kPinChunks], c->stream);
+    };
+    cudaError_t e = cudaSuccess;
+    for (size_t i = 0; i < std::min(n, kPinChunks) && e == cudaSuccess; ++i) e = fetch(i);
+    for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
+        e = cudaEventSynchronize(c->pin_ready[i % kPinChunks]);
+        if (e != cudaSuccess) break;
+        memcpy(dst[i / per] + i % per * kPinChunk, ring.p + i % kPinChunks * kPinChunk, len(i));
+        if (i + kPinChunks < n) e = fetch(i + kPinChunks);
+    }
+    if (e != cudaSuccess) cudaStreamSynchronize(c->stream);  // no copy into the ring once it is given back
+    CK(e);
+    return HGPM_OK;
+}
+
 extern "C" int hgpm_load_state_device(hgpm_ctx* c, const float* x, const float* v) {
     if (!c || !x || !v) return HGPM_ERR_ARG;
     CK(launch_load_state(x, v, c->part, c->np, c->blk, c->ng, c->stream));
@@ -571,9 +678,7 @@ extern "C" int hgpm_store_state(hgpm_ctx* c, float* x, float* v) {
     if (rc) return rc;
     rc = hgpm_store_state_device(c, c->stage, c->stage + 3 * c->npart);
     if (rc) return rc;
-    size_t bytes = c->npart * 3 * sizeof(float);
-    CK(cudaMemcpyAsync(x, c->stage, bytes, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(v, c->stage + 3 * c->npart, bytes, cudaMemcpyDeviceToHost, c->stream));
+    if ((rc = copy_out(c, x, v))) return rc;
     return sync_check(c);
 }
 

@@ -4,6 +4,8 @@ Bars: cell indices bit-exact; density bit-exact run to run and within 1e-6
 of the oracle's max; forces within FIELD_RTOL (1e-5) of the oracle's max;
 positions/velocities after a phase within float rounding.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -13,6 +15,7 @@ from tests.helpers import FIELD_RTOL, lattice_state, params_text, rel_max_err
 
 pytestmark = pytest.mark.gpu
 
+F = ctypes.POINTER(ctypes.c_float)
 SIZES = [16, 24, 32, 40, 48, 64, 80, 96, 120, 128, 160, 200]
 
 
@@ -605,3 +608,22 @@ def test_one_kernel_solve_equals_passes(ng, np_side):
         got.append((first, rho, xo, vo))
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("np_side", [32, 40, 64, 96])
+def test_store_to_pageable_and_pinned_arrays(np_side):
+    """The state stored into pageable arrays (in chunks; 32 below one chunk, 40
+    and 96 with a part of one left) and into page-locked ones is the state on
+    the device."""
+    import torch
+
+    n = np_side ** 3
+    x, v = lattice_state(np_side, np_side, disp=1.0, vel=0.5, seed=4)
+    with make(np_side) as s:
+        s.load_state(x, v)
+        for _ in range(2):
+            xp, vp = s.store_state()
+            assert np.array_equal(xp, x) and np.array_equal(vp, v)
+        xl, vl = (torch.full((n, 3), -7.0).pin_memory() for _ in range(2))
+        assert s.L.hgpm_store_state(s._h, ctypes.cast(xl.data_ptr(), F), ctypes.cast(vl.data_ptr(), F)) == 0
+        assert np.array_equal(xl.numpy(), x) and np.array_equal(vl.numpy(), v)
