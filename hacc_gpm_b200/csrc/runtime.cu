@@ -605,7 +605,7 @@ static int copy_out(hgpm_ctx* c, float* x, float* v) {
     const size_t bytes = c->npart * 3 * sizeof(float);
     char* dst[2] = {(char*)x, (char*)v};
     const char* src[2] = {(const char*)c->stage, (const char*)(c->stage + 3 * c->npart)};
-    bool pageable = bytes >= kPinChunk;  // below it the driver's copy is as fast
+    bool pageable = bytes >= kPinChunk;  // (below, there is nothing to overlap)
     for (int a = 0; a < 2 && pageable; ++a) {
         cudaPointerAttributes at;
         CK(cudaPointerGetAttributes(&at, dst[a]));
