@@ -553,7 +553,8 @@ def test_solve_of_large_sides_matches_double_fft(ng, np_side):
 
 
 @pytest.mark.parametrize("ng,np_side,choice", [(32, 32, "9"), (32, 32, "8"), (64, 64, "8"), (40, 40, "4"), (64, 32, "1"),
-                                               (64, 32, "0"), (128, 16, "0"), (48, 96, None)])
+                                               (64, 32, "0"), (128, 16, "0"), (48, 96, None), (128, 128, "8"),
+                                               (160, 160, "8")])
 def test_dense_cells_reach_the_solve(ng, np_side, choice, monkeypatch):
     """Half the particles in a few cells, far from their blocks' windows and
     thousands of units of weight in each: the forces match the oracle's on the
