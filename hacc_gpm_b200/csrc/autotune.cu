@@ -250,7 +250,7 @@ extern "C" int hgpm_autotune(hgpm_ctx* c, int reps, int store, int choices[HGPM_
     int rc = hgpm_deposit(c);
     c->kick_choice = kick0;
     if (rc) return rc;
-    rc = hgpm_solve_gradient(c);
+    rc = ctx_solve_passes(c);  // whatever the side: the spectrum it leaves is read below
     if (rc) return rc;
     rc = hgpm_sync(c);
     if (rc) return rc;
@@ -298,10 +298,14 @@ extern "C" int hgpm_autotune(hgpm_ctx* c, int reps, int store, int choices[HGPM_
     }
     c->kick_choice = pick[HGPM_TUNE_KICK];
     // the potential is the current one; the force grid's space now holds the
-    // paired potential
+    // paired potential, or the grid again where the kick gathers it
+    const bool grid = !kick_uses_phi(c->kick_choice);
+    if (grid)
+        CK(launch_gradient(ng, reinterpret_cast<float*>(c->fspec + (size_t)ng * ng * c->zs),
+                           reinterpret_cast<float4*>(c->force), c->stream));
     c->phi_valid = true;
-    c->force_valid = false;
-    c->phi2_valid = true;
+    c->force_valid = grid;
+    c->phi2_valid = !grid;
     CK(cudaStreamSynchronize(c->stream));
     if (choices)
         for (int k = 0; k < HGPM_TUNE_KNOBS; ++k) choices[k] = pick[k];

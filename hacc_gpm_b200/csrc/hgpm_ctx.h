@@ -150,6 +150,9 @@ static_assert(PH_PK + 1 == HGPM_NPHASE, "phase ids");
 int ctx_set_rl_tables(hgpm_ctx* c);
 // Unit-mass CIC weight scale (ng/np)^3 of pm_actions.cpp:229-230.
 float ctx_cic_mass(int ng, int np);
+// hgpm_solve_gradient as separate passes on every side, so that the potential's
+// spectrum is left in fspec (the one-kernel solve of small boxes forms none).
+int ctx_solve_passes(hgpm_ctx* c);
 // Apply the autotuner's cached entry for this context's size and device
 // (autotune.cu); returns 1 if one was applied.
 int ctx_apply_tuned(hgpm_ctx* c);

@@ -875,7 +875,7 @@ static bool solve_in_one_kernel(const hgpm_ctx* c) {
 extern "C" int hgpm_solve_gradient(hgpm_ctx* c) {
     if (!c) return HGPM_ERR_ARG;
     if (!c->rho_dirty) return fail(c, HGPM_ERR_STATE, "no deposited density (call hgpm_deposit first)");
-    const int ng = c->ng, M = ng / 2;
+    const int ng = c->ng;
     const double coeff = 0.5 / ((double)ng * ng * ng);
     if (solve_in_one_kernel(c)) {
         PhaseScope ps(c, PH_POISSON);
@@ -886,6 +886,12 @@ extern "C" int hgpm_solve_gradient(hgpm_ctx* c) {
         count(c, PH_POISSON, 1);
         return HGPM_OK;
     }
+    return ctx_solve_passes(c);
+}
+
+int ctx_solve_passes(hgpm_ctx* c) {
+    const int ng = c->ng, M = ng / 2;
+    const double coeff = 0.5 / ((double)ng * ng * ng);
     int rc = forward_zy(c);
     if (rc) return rc;
     const size_t cs = (size_t)ng * ng * c->zs;

@@ -628,3 +628,36 @@ def test_store_to_pageable_and_pinned_arrays(np_side):
         xl, vl = (torch.full((n, 3), -7.0).pin_memory() for _ in range(2))
         assert s.L.hgpm_store_state(s._h, ctypes.cast(xl.data_ptr(), F), ctypes.cast(vl.data_ptr(), F)) == 0
         assert np.array_equal(xl.numpy(), x) and np.array_equal(vl.numpy(), v)
+
+
+@pytest.mark.parametrize("ng", [16, 24, 32, 40, 48])
+@pytest.mark.parametrize("reps", [2, 40])
+def test_autotune_leaves_the_current_potential(ng, reps, monkeypatch):
+    """Straight after hgpm_autotune the context holds the state it had, the
+    potential of that state, and a kick without another solve moves the
+    particles as in a context that was never tuned, bit for bit: at the sides
+    that solve in one kernel too, whatever the repetitions."""
+    for k in ("HGPM_DEPOSIT", "HGPM_KICK", "HGPM_NO_TMA", "HGPM_XTMA", "HGPM_PLANE"):
+        monkeypatch.delenv(k, raising=False)
+    monkeypatch.setenv("HGPM_NO_TUNE_CACHE", "1")
+    x, v = lattice_state(ng, ng, disp=1.5, vel=0.2, seed=ng)
+    got = []
+    for tune, force_first in ((False, False), (True, False), (True, True)):
+        with make(ng) as s:
+            s.load_state(x, v)
+            if tune:
+                s.autotune(reps=reps)
+                xt, vt = s.store_state()
+                assert np.array_equal(xt, x) and np.array_equal(vt, v)
+            else:
+                s.cic()
+                s.solve_gradient()
+            if force_first:
+                s.get_force()
+            s.kick_drift(0.0123, 1.7, 0.3, 0.25, 2)
+            xo, vo = s.store_state()
+            got.append((s.get_force(), xo, vo))
+    assert not np.array_equal(got[0][2], v)
+    for a in got[1:]:
+        for p, q in zip(got[0], a):
+            assert np.array_equal(p, q)
