@@ -66,6 +66,7 @@ struct EnsClass {
     cudaGraphExec_t exec = nullptr; // one step of this class alone (hgpm_ens_step_class)
     std::vector<hgpm_ctx*> views;
     std::vector<int> in_use;   // host: slot started and not released
+    std::vector<int> left;     // host: steps of its run not yet queued
 };
 
 }  // namespace
@@ -204,6 +205,7 @@ static int make_class(hgpm_ensemble* E, EnsClass& k, int priority) {
     E->launches += 1;
     ECK(cudaStreamSynchronize(E->stream));
     k.in_use.assign(S, 0);
+    k.left.assign(S, 0);
     k.views.assign(S, nullptr);
     return HGPM_OK;
 }
@@ -416,6 +418,7 @@ extern "C" int hgpm_ens_start(hgpm_ensemble* E, int ci, int slot, hgpm_timestepp
     ECK(cudaMemcpyAsync(k.d_nsteps + slot, st + 2, 4, cudaMemcpyHostToDevice, E->stream));
     ECK(cudaMemcpyAsync(k.d_active + slot, st + 0, 4, cudaMemcpyHostToDevice, E->stream));
     k.in_use[slot] = 1;
+    k.left[slot] = nsteps;
     k.h_mirror[slot] = 1;
     k.h_mirror[k.nslots + slot] = 0;
     return HGPM_OK;
@@ -428,6 +431,7 @@ extern "C" int hgpm_ens_release(hgpm_ensemble* E, int ci, int slot) {
     if (k.in_use[slot] && k.h_mirror[slot])
         return efail(E, HGPM_ERR_STATE, "class %d slot %d still has steps to run", ci, slot);
     k.in_use[slot] = 0;
+    k.left[slot] = 0;
     return HGPM_OK;
 }
 
@@ -438,12 +442,16 @@ static int step_kernels(const hgpm_ensemble* E, const EnsClass& k) {
            kick_kernels(E->kick_choice, k.np, k.ng);
 }
 
-// The slots with steps to run are about to hold the potential that form of
-// step leaves: their views form a force grid from its spectrum on demand.
-static void mark_stepped(EnsClass& k, bool pair, bool grid) {
+// nsteps steps of the class are about to be queued: the slots with steps to run
+// will hold the potential that form of step leaves, and their views form a
+// force grid from it on demand.  By the steps queued, not by h_mirror, which is
+// as old as the last sync: a slot that has run out keeps what its view holds.
+static void mark_stepped(EnsClass& k, int nsteps, bool pair, bool grid) {
+    if (nsteps == 0) return;
     for (int s = 0; s < k.nslots; ++s) {
+        if (k.left[s] == 0) continue;
+        k.left[s] -= std::min(k.left[s], nsteps);
         hgpm_ctx* v = k.views[s];
-        if (!v || !k.in_use[s] || !k.h_mirror[s]) continue;
         v->phi2_valid = pair;
         v->phi_valid = !pair;
         v->force_valid = grid;
@@ -610,9 +618,9 @@ extern "C" int hgpm_ens_use_graph(hgpm_ensemble* E, int on) {
 
 extern "C" int hgpm_ens_step(hgpm_ensemble* E, int nsteps) {
     if (!E || nsteps < 0) return HGPM_ERR_ARG;
-    if (nsteps > 0)
-        for (auto& k : E->cls) mark_stepped(k, multi_ok(E) || kick_uses_phi2(E->kick_choice),
-                                            !multi_ok(E) && !kick_uses_phi(E->kick_choice));
+    for (auto& k : E->cls)
+        mark_stepped(k, nsteps, multi_ok(E) || kick_uses_phi2(E->kick_choice),
+                     !multi_ok(E) && !kick_uses_phi(E->kick_choice));
     if (E->use_graph) {
         if (!E->exec) {
             // the graph covers every class (idle slots cost one early-exit CTA
@@ -665,7 +673,7 @@ extern "C" int hgpm_ens_step_class(hgpm_ensemble* E, int ci, int nsteps) {
     if (rc) return rc;
     if (nsteps < 0) return efail(E, HGPM_ERR_ARG, "nsteps < 0");
     EnsClass& k = E->cls[ci];
-    if (nsteps > 0) mark_stepped(k, kick_uses_phi2(E->kick_choice), !kick_uses_phi(E->kick_choice));
+    mark_stepped(k, nsteps, kick_uses_phi2(E->kick_choice), !kick_uses_phi(E->kick_choice));
     ECK(cudaEventRecord(k.setup, E->stream));
     ECK(cudaStreamWaitEvent(k.stream, k.setup, 0));
     if (E->use_graph) {

@@ -142,3 +142,47 @@ def test_serving_mix_equals_alone():
     for r in alone:
         g = by_tag[r.tag].result
         assert np.array_equal(g["n"], r.result["n"]) and np.array_equal(g["P"], r.result["P"])
+
+
+@pytest.mark.parametrize("per_class", [False, True])
+@pytest.mark.parametrize("classes,multi", [([(24, 24, 2), (40, 40, 2)], False), ([(32, 32, 2), (48, 48, 2)], True),
+                                           ([(32, 32, 2), (48, 48, 2)], False)])
+def test_finished_slot_keeps_its_force_grid(classes, multi, per_class):
+    """A slot that has run its steps keeps the potential of its last one while
+    others step on, whether or not its force grid was asked for in between and
+    without a sync; the slot that steps on has the grid of its own last step."""
+    def box(ng, i, nsteps):
+        return E.Box(ng=ng, rl=float(ng), seed=7 + i, nsteps=nsteps, n_total=100, z_ini=50.0)
+
+    boxes = [(ci, si, box(c[0], 2 * ci + si, (1, 4)[si])) for ci, c in enumerate(classes) for si in (0, 1)]
+    E.prepare_tables([b for _, _, b in boxes])
+    alone = {}
+    for ci, si, b in boxes:
+        with H.Simulation(b.params()) as s:
+            s.generate_ic(b.table, b.k_delta)
+            s.run_steps(E._ts_for(b.params()), b.nsteps)
+            alone[ci, si] = s.get_force()
+    with E.Ensemble(classes, multi=multi) as ens:
+        for ci, si, b in boxes:
+            ens.slot(ci, si, b.params()).generate_ic(b.table, b.k_delta)
+            ens.start(ci, si, E._ts_for(b.params()), b.nsteps)
+
+        def step(n):
+            if not per_class:
+                ens.step(n)
+                return
+            for ci in range(len(classes)):
+                ens.step_class(ci, n)
+            for ci in range(len(classes)):
+                while not ens.class_done(ci):
+                    pass
+
+        step(1)
+        for n in (1, 2, 3):  # the second slots end with the 4th step
+            for ci in range(len(classes)):
+                assert np.array_equal(ens.views[ci, 0].get_force(), alone[ci, 0])
+            step(n)
+        for ci in range(len(classes)):
+            for si in (0, 1):
+                assert np.array_equal(ens.views[ci, si].get_force(), alone[ci, si])
+        ens.sync()
