@@ -1666,7 +1666,10 @@ static cudaError_t func_attr_once(const void* func, int bytes, int threads) {
     std::lock_guard<std::mutex> g(mu);
     auto it = done.find({dev, func});
     if (it != done.end() && it->second >= bytes) return cudaSuccess;
-    if (bytes > 48 * 1024) {
+    cudaFuncAttributes fa;
+    if ((e = cudaFuncGetAttributes(&fa, func)) != cudaSuccess) return e;
+    // without being asked for, a CTA's static and dynamic memory together end at 48 KB
+    if (bytes + (int)fa.sharedSizeBytes > 48 * 1024) {
         e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return e;
     }
@@ -1676,8 +1679,6 @@ static cudaError_t func_attr_once(const void* func, int bytes, int threads) {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, threads, bytes);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
         if (e != cudaSuccess) return e;
-        cudaFuncAttributes fa;
-        if ((e = cudaFuncGetAttributes(&fa, func)) != cudaSuccess) return e;
         // the smallest of the SM's splits that holds them (1 KB a CTA is the
         // system's), named by a percentage that rounds up to it
         const int each = (bytes + (int)fa.sharedSizeBytes + 1024 + 127) / 128 * 128;

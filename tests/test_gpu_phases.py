@@ -661,3 +661,27 @@ def test_autotune_leaves_the_current_potential(ng, reps, monkeypatch):
     for a in got[1:]:
         for p, q in zip(got[0], a):
             assert np.array_equal(p, q)
+
+
+def test_power_spectrum_with_every_number_of_bins():
+    """P(k) runs with any number of bins, also where the tile and the
+    histograms come to just under 48 KB.  In a process of its own and in
+    ascending order: what a kernel may use is asked for once, so a larger
+    spectrum before would hide a smaller one that is refused."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    code = """
+from tests.helpers import lattice_state, params_text
+import hacc_gpm_b200 as H
+for ng, bins in ((48, range(1, 500, 3)), (64, range(1, 500, 3)), (200, range(190, 230)), (256, range(110, 140)),
+                 (320, range(340, 370)), (512, range(110, 140))):
+    with H.Simulation(H.parse_params(params_text(ng, 32))) as s:
+        s.load_state(*lattice_state(32, ng))
+        total = {int(s.power_spectrum(n)[2].sum()) for n in bins}
+        assert len(total) == 1, (ng, total)
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
