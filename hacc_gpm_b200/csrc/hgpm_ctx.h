@@ -20,6 +20,8 @@ struct PhaseRec {
 };
 
 constexpr size_t kPinChunks = 4, kPinChunk = 512 << 10;  // copy_out's ring
+constexpr size_t kPinPays = 128 << 20;                   // and when a context allocates one
+constexpr int kPinStores = 3;
 
 struct hgpm_ctx {
     hgpm_params p;
@@ -67,6 +69,7 @@ struct hgpm_ctx {
     int kick_choice = 0;
     float* stage = nullptr;     // AoS float3 x, v staging (lazy)
     cudaEvent_t pin_ready[kPinChunks] = {};  // copy_out's chunks (lazy)
+    int pin_stores = 0;         // stores that a ring is for
     bool pins = false;          // counted among the users of the page-locked rings
     double* pk_part = nullptr;  // P(k) partial sums (lazy)
     unsigned long long* pk_pcnt = nullptr;

@@ -3,6 +3,8 @@
 // context, and the phase sequencing that launches the kernels of
 // particles.cu and the fft_*.cu passes on the context's stream.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <cmath>
 #include <cstdarg>
@@ -540,9 +542,9 @@ static int ensure_stage(hgpm_ctx* c) {
     return HGPM_OK;
 }
 
-// Page-locked rings for copy_out, shared by the contexts: a ring costs 3 ms to
-// allocate, so a context takes one for the length of a copy.  At most
-// kPinKeep are kept between copies, and none once the last context that
+// Page-locked rings for copy_out, shared by the contexts: a ring costs 1 to 3 ms
+// to allocate and 0.4 to free, so a context takes one for the length of a copy.
+// At most kPinKeep are kept between copies, and none once the last context that
 // copied is gone.
 namespace {
 constexpr int kPinKeep = 4;
@@ -552,7 +554,8 @@ int pin_nfree = 0, pin_users = 0;
 
 struct PinRing {
     char* p = nullptr;
-    explicit PinRing(bool want) {
+    // one that is kept, or (make) a new one
+    PinRing(bool want, bool make) {
         if (!want) return;
         {
             std::lock_guard<std::mutex> g(pin_mutex);
@@ -561,7 +564,7 @@ struct PinRing {
                 return;
             }
         }
-        if (cudaHostAlloc((void**)&p, kPinChunks * kPinChunk, cudaHostAllocPortable) != cudaSuccess) {
+        if (make && cudaHostAlloc((void**)&p, kPinChunks * kPinChunk, cudaHostAllocPortable) != cudaSuccess) {
             cudaGetLastError();
             p = nullptr;
         }
@@ -596,49 +599,77 @@ static void pin_leave() {
     while (n > 0) cudaFreeHost(drop[--n]);
 }
 
-// The staged state to the caller's arrays.  Into pageable memory the driver
-// copies 6.3 MB (64^3) in 1.02 ms; through a ring of page-locked chunks, the
-// next ones on their way while the host copies one out, it is the host's copy
-// alone (0.35 ms; five steps of 64^3 between host arrays 2.41 -> 1.70 ms).
-// Page-locked (or device) destinations are copied directly.
+// Whether p is ordinary host memory that has yet to get its pages, as a new
+// array of some size has (by 8 pages of it), and may be written to.
+static bool unmapped_pages(const void* p, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return false;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t a = (uintptr_t)p / page, last = ((uintptr_t)p + bytes - 1) / page;
+    for (int k = 0; k < 8; ++k) {
+        void* q = (void*)((a + (last - a) * k / 7) * page);
+        unsigned char in = 1;
+        if (mincore(q, page, &in) != 0) return false;
+        if (!(in & 1)) return madvise(q, page, MADV_POPULATE_WRITE) == 0;
+    }
+#else
+    (void)p, (void)bytes;
+#endif
+    return false;
+}
+
+// The staged state to the caller's arrays: by the driver, or, into pageable
+// arrays whose pages are yet to come, through a ring of page-locked chunks, the
+// next ones on their way while the host copies one out, which takes the page
+// faults in less time than the driver.  ms a store, ring / driver, new pages:
+// 64^3 1.77 / 3.1, 128^3 7.9 / 11.3, 256^3 64 / 79, 512^3 620 / 735; arrays that
+// have their pages: 0.44 / 0.39, 3.3 / 2.5, 35 / 19, 280 / 160, so these are
+// left to the driver, as page-locked and device destinations are.  A store of
+// 128 MB pays for the ring it allocates; smaller ones get one at a context's
+// third, when what the driver took longer for has come to as much.
 static int copy_out(hgpm_ctx* c, float* x, float* v) {
-    const size_t bytes = c->npart * 3 * sizeof(float);
+    const size_t bytes = c->npart * 3 * sizeof(float), n = (bytes + kPinChunk - 1) / kPinChunk;
     char* dst[2] = {(char*)x, (char*)v};
     const char* src[2] = {(const char*)c->stage, (const char*)(c->stage + 3 * c->npart)};
-    bool pageable = bytes >= kPinChunk;  // (below, there is nothing to overlap)
-    for (int a = 0; a < 2 && pageable; ++a) {
-        cudaPointerAttributes at;
-        CK(cudaPointerGetAttributes(&at, dst[a]));
-        pageable = at.type == cudaMemoryTypeUnregistered;
-    }
-    if (pageable && !c->pins) {
+    bool ringed[2] = {};
+    for (int a = 0; a < 2 && bytes >= kPinChunk; ++a)  // (below, there is nothing to overlap)
+        ringed[a] = unmapped_pages(dst[a], bytes);
+    const bool any = ringed[0] || ringed[1];
+    if (any && !c->pins) {
         for (auto& e : c->pin_ready)
             if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         pin_join();
         c->pins = true;
     }
-    PinRing ring(pageable);
-    if (!ring.p) {
-        for (int a = 0; a < 2; ++a) CK(cudaMemcpyAsync(dst[a], src[a], bytes, cudaMemcpyDeviceToHost, c->stream));
-        return HGPM_OK;
+    if (any && c->pin_stores < kPinStores) ++c->pin_stores;
+    PinRing ring(any, 2 * bytes >= kPinPays || c->pin_stores == kPinStores);
+    auto len = [&](size_t i) { return std::min(kPinChunk, bytes - i * kPinChunk); };
+    for (int a = 0; a < 2; ++a) {
+        if (!ringed[a] || !ring.p) {
+            CK(cudaMemcpyAsync(dst[a], src[a], bytes, cudaMemcpyDeviceToHost, c->stream));
+            continue;
+        }
+        auto fetch = [&](size_t i) {
+            cudaError_t e = cudaMemcpyAsync(ring.p + i % kPinChunks * kPinChunk, src[a] + i * kPinChunk, len(i),
+                                            cudaMemcpyDeviceToHost, c->stream);
+            return e != cudaSuccess ? e : cudaEventRecord(c->pin_ready[i % kPinChunks], c->stream);
+        };
+        cudaError_t e = cudaSuccess;
+        for (size_t i = 0; i < std::min(n, kPinChunks) && e == cudaSuccess; ++i) e = fetch(i);
+        for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
+            e = cudaEventSynchronize(c->pin_ready[i % kPinChunks]);
+            if (e != cudaSuccess) break;
+            memcpy(dst[a] + i * kPinChunk, ring.p + i % kPinChunks * kPinChunk, len(i));
+            if (i + kPinChunks < n) e = fetch(i + kPinChunks);
+        }
+        if (e != cudaSuccess) cudaStreamSynchronize(c->stream);  // no copy into the ring once it is given back
+        CK(e);
     }
-    const size_t per = (bytes + kPinChunk - 1) / kPinChunk, n = 2 * per;
-    auto len = [&](size_t i) { return std::min(kPinChunk, bytes - i % per * kPinChunk); };
-    auto fetch = [&](size_t i) {
-        cudaError_t e = cudaMemcpyAsync(ring.p + i % kPinChunks * kPinChunk, src[i / per] + i % per * kPinChunk, len(i),
-                                        cudaMemcpyDeviceToHost, c->stream);
-        return e != cudaSuccess ? e : cudaEventRecord(c->pin_ready[i % kPinChunks], c->stream);
-    };
-    cudaError_t e = cudaSuccess;
-    for (size_t i = 0; i < std::min(n, kPinChunks) && e == cudaSuccess; ++i) e = fetch(i);
-    for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
-        e = cudaEventSynchronize(c->pin_ready[i % kPinChunks]);
-        if (e != cudaSuccess) break;
-        memcpy(dst[i / per] + i % per * kPinChunk, ring.p + i % kPinChunks * kPinChunk, len(i));
-        if (i + kPinChunks < n) e = fetch(i + kPinChunks);
-    }
-    if (e != cudaSuccess) cudaStreamSynchronize(c->stream);  // no copy into the ring once it is given back
-    CK(e);
     return HGPM_OK;
 }
 

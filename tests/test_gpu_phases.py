@@ -685,3 +685,33 @@ for ng, bins in ((48, range(1, 500, 3)), (64, range(1, 500, 3)), (200, range(190
 """
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("np_side", [40, 64, 96])
+@pytest.mark.parametrize("new", [(True, True), (True, False), (False, True), (False, False)])
+def test_store_to_arrays_with_and_without_pages(np_side, new):
+    """Stores into arrays that have no pages yet (through page-locked chunks from
+    a context's third such store on) and into arrays that have them (by the
+    driver), one of each too, give the state on the device and leave the bytes
+    around the arrays alone."""
+    import mmap
+
+    n = np_side ** 3
+    x, v = lattice_state(np_side, np_side, disp=1.0, vel=0.5, seed=4)
+    with make(np_side) as s:
+        s.load_state(x, v)
+        for _ in range(5):
+            maps, out = [], []
+            for fresh in new:
+                m = mmap.mmap(-1, 12 * n + 8192, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+                a = np.frombuffer(m, np.float32)
+                if not fresh:
+                    a[:] = -7.0
+                maps.append((m, a))
+                out.append(a[5:5 + 3 * n])
+            ptr = [ctypes.cast(a.ctypes.data, F) for a in out]
+            assert s.L.hgpm_store_state(s._h, *ptr) == 0
+            assert np.array_equal(out[0].reshape(n, 3), x) and np.array_equal(out[1].reshape(n, 3), v)
+            for fresh, (m, a) in zip(new, maps):
+                around = 0.0 if fresh else -7.0
+                assert (a[:5] == around).all() and (a[5 + 3 * n:] == around).all()
