@@ -207,8 +207,9 @@ extern "C" int hgpm_autotune(hgpm_ctx* c, int reps, int store, int choices[HGPM_
     CK(launch_zfwd_rho(ng, c->rho64, c->spec, c->zs, mean, c->tw_ng, c->stream));
     // y pass: 1 = TMA-fed, 0 = plain (in place on the spectrum: timing only;
     // the spectrum is rebuilt below)
+    double yms[2], xms[3];
     {
-        double ms[2];
+        double* ms = yms;
         for (int t = 0; t < 2; ++t) {
             ms[t] = time_launches(c, reps, [&] {
                 return t ? launch_strided_tma(ng, false, false, c->spec, M + 1, c->zs, 0, 1, c->tw_ng, c->d_err + 1,
@@ -222,9 +223,9 @@ extern "C" int hgpm_autotune(hgpm_ctx* c, int reps, int store, int choices[HGPM_
         pms[HGPM_TUNE_YPASS] = ms[pick[HGPM_TUNE_YPASS]];
     }
     // x pass with the Green's function: 1 = TMA-fed, 0 and 2 = the line tiles
+    const double coeff = 0.5 / ((double)ng * ng * ng);
     {
-        double ms[3];
-        const double coeff = 0.5 / ((double)ng * ng * ng);
+        double* ms = xms;
         for (int t = 0; t < 3; ++t) {
             ms[t] = time_launches(c, reps, [&] {
                 if (t == 1)
@@ -283,18 +284,49 @@ extern "C" int hgpm_autotune(hgpm_ctx* c, int reps, int store, int choices[HGPM_
             CK(e);
             if (!kick_uses_phi(i)) ms[i] += grad_ms;
         }
+        // A side whose solve can run as one kernel runs so with the paired kick
+        // at y pass 0 and an x pass other than 1.  Its passes alone, 2-3 us
+        // each, say nothing of that kernel (a y pick of 1 by 2 % gave up 10 us a
+        // step at 32^3), so it is weighed against the five passes of the picks.
+        // (The accumulator is empty and the spectrum not read any more.)
+        const bool small = solve_small_supported(ng);
+        double one_ms = 0.0, passes_ms = 0.0;  // the latter but for the last pass
+        if (small) {
+            passes_ms = 2 * pms[HGPM_TUNE_YPASS] + pms[HGPM_TUNE_XPASS] + time_launches(c, reps, [&] {
+                return launch_zfwd_rho(ng, c->rho64, c->spec, c->zs, mean, c->tw_ng, c->stream);
+            }, &e);
+            CK(e);
+            one_ms = time_launches(c, reps, [&] {
+                return launch_solve_small(ng, c->rho64, c->force, mean, c->tw_ng, c->cosq, coeff, c->stream);
+            }, &e);
+            CK(e);
+        }
         // the paired potential (in the force grid's space, so after the
         // candidates that gather the grid), charged the extra bytes its z
-        // pass writes over the plain one
+        // pass writes over the plain one; or, where its solve is one kernel,
+        // the others are charged what theirs takes over that
         const double z2 = time_launches(c, reps, [&] { return launch_zinv_pair(ng, c->fspec, c->force, c->zs, c->tw_ng, c->stream); }, &e);
         CK(e);
+        const double solves[2] = {one_ms, passes_ms + z2};
+        const bool one = small && hgpm_tune_pick(solves, 2, 0, tol) == 0;
         for (int i = 0; i < n; ++i) {
-            if (!kick_uses_phi2(i)) continue;
-            ms[i] = time_kick(i, c->force) + (z2 - z1);
-            CK(e);
+            if (kick_uses_phi2(i)) {
+                ms[i] = time_kick(i, c->force) + (one ? 0.0 : z2 - z1);
+                CK(e);
+            } else if (one) {
+                ms[i] += passes_ms + z1 - one_ms;
+            }
         }
         pick[HGPM_TUNE_KICK] = hgpm_tune_pick(ms.data(), n, kick_default(np, ng), tol);
         pms[HGPM_TUNE_KICK] = ms[pick[HGPM_TUNE_KICK]];
+        if (one && kick_uses_phi2(pick[HGPM_TUNE_KICK])) {
+            pick[HGPM_TUNE_YPASS] = 0;
+            if (pick[HGPM_TUNE_XPASS] == 1) pick[HGPM_TUNE_XPASS] = 2;
+            pms[HGPM_TUNE_YPASS] = yms[0];
+            pms[HGPM_TUNE_XPASS] = xms[pick[HGPM_TUNE_XPASS]];
+            c->tma = false;
+            c->xmode = pick[HGPM_TUNE_XPASS];
+        }
     }
     c->kick_choice = pick[HGPM_TUNE_KICK];
     // the potential is the current one; the force grid's space now holds the

@@ -715,3 +715,26 @@ def test_store_to_arrays_with_and_without_pages(np_side, new):
             for fresh, (m, a) in zip(new, maps):
                 around = 0.0 if fresh else -7.0
                 assert (a[:5] == around).all() and (a[5 + 3 * n:] == around).all()
+
+
+@pytest.mark.parametrize("ng", [16, 24, 32])
+def test_autotune_weighs_the_one_kernel_solve(ng, monkeypatch):
+    """A tuned small box steps in three kernels, as an untuned one does: the
+    deposit, the whole solve and the kick.  What the tuner finds for the y pass,
+    the x pass or another kick alone does not give up the one-kernel solve,
+    which takes about half of what five passes take at these sides."""
+    for k in ("HGPM_DEPOSIT", "HGPM_KICK", "HGPM_NO_TMA", "HGPM_XTMA", "HGPM_PLANE"):
+        monkeypatch.delenv(k, raising=False)
+    monkeypatch.setenv("HGPM_NO_TUNE_CACHE", "1")
+    x, v = lattice_state(ng, ng, disp=1.0, vel=0.2, seed=ng)
+    for _ in range(8):
+        with make(ng) as s:
+            s.load_state(x, v)
+            picks = s.autotune(reps=10)
+            assert all(p["ms"] > 0 for p in picks.values())
+            s.kernel_launches(reset=True)
+            s.cic()
+            s.solve_gradient()
+            s.kick_drift(0.0123, 1.7, 0.3, 0.25, 2)
+            assert s.kernel_launches() <= 4, picks  # a windowed deposit is two
+            assert picks["kick"]["choice"] == 7 and picks["y_pass"]["choice"] == 0 and picks["x_pass"]["choice"] != 1
