@@ -362,7 +362,9 @@ int hgpm_tuned_choices(const hgpm_ctx* ctx, int choices[HGPM_TUNE_KNOBS]);
  * unless the default `def` is within a fraction `tol` of it.              */
 int hgpm_tune_pick(const double* ms, int n, int def, double tol);
 /* Cache file access (host only): lookup returns 1 and fills choices when a
- * line for (device, sms, ng, np) exists (the last one wins), else 0;
+ * line for (device, sms, ng, np) exists (the last one wins), else 0; lines of
+ * the format's first version, whose numbers stood for other kernels, are not
+ * applied (tune again);
  * store appends one line.  device: one token without blanks.              */
 int hgpm_tune_cache_lookup(const char* path, const char* device, int sms, int ng, int np,
                            int choices[HGPM_TUNE_KNOBS]);

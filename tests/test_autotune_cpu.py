@@ -62,3 +62,14 @@ def test_cache_rejects_blank_device_names(built_lib, tmp_path):
 
 def test_binding_names_the_knobs():
     assert binding.TUNE_NAMES == ("deposit", "kick", "y_pass", "x_pass") and binding.TUNE_KNOBS == 4
+
+
+def test_cache_lines_of_the_first_version_are_not_applied(built_lib, tmp_path):
+    """Their choices were timed against other kernels under the same numbers."""
+    f = tmp_path / "tune.txt"
+    f.write_text("v1 NVIDIA_B200 148 32 32 8 5 1 2 0.0100 0.0100 0.0030 0.0030\n")
+    assert _lookup(built_lib, f, "NVIDIA_B200", 148, 32, 32)[0] == 0
+    assert _store(built_lib, f, "NVIDIA_B200", 148, 32, 32, [9, 7, 0, 2]) == 0
+    with open(f, "a") as fh:
+        fh.write("v1 NVIDIA_B200 148 32 32 8 5 1 2 0.0100 0.0100 0.0030 0.0030\n")
+    assert _lookup(built_lib, f, "NVIDIA_B200", 148, 32, 32) == (1, [9, 7, 0, 2])
