@@ -738,3 +738,28 @@ def test_autotune_weighs_the_one_kernel_solve(ng, monkeypatch):
             s.kick_drift(0.0123, 1.7, 0.3, 0.25, 2)
             assert s.kernel_launches() <= 4, picks  # a windowed deposit is two
             assert picks["kick"]["choice"] == 7 and picks["y_pass"]["choice"] == 0 and picks["x_pass"]["choice"] != 1
+
+
+@pytest.mark.parametrize("ng,np_side", [(16, 16), (24, 24), (32, 32), (40, 40), (32, 64)])
+@pytest.mark.parametrize("var,values", [("HGPM_XTMA", ("1", "2")), ("HGPM_NO_TMA", ("0", "1"))])
+def test_line_tiles_of_small_sides_equal_tma(ng, np_side, var, values, monkeypatch):
+    """The separate y and x passes in line tiles at the sides whose solve is one
+    kernel otherwise: with the phases timed the passes run, and they move the
+    particles as the TMA-fed ones do, bit for bit."""
+    rng = np.random.default_rng(ng)
+    x = rng.random((np_side ** 3, 3), dtype=np.float32) * np.float32(ng * (1 - 2 ** -20))
+    v = rng.standard_normal((np_side ** 3, 3), dtype=np.float32)
+    out = []
+    for value in values:
+        monkeypatch.setenv(var, value)
+        with make(ng, np_side) as s:
+            s.enable_timing(True)
+            s.load_state(x, v)
+            s.kernel_launches(reset=True)
+            s.cic()
+            s.solve_gradient()
+            assert s.kernel_launches() >= 6  # a deposit and five passes
+            s.kick_drift(0.0123, 1.7, 0.3, 0.25, 2)
+            out.append(s.store_state())
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    assert not np.array_equal(out[0][1], v)
