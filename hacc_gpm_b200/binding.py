@@ -166,6 +166,7 @@ def lib() -> C.CDLL:
         "hgpm_tune_cache_store": (C.c_int, [C.c_char_p, C.c_char_p, C.c_int, C.c_int, C.c_int, P(C.c_int),
                                             P(C.c_double)]),
         "hgpm_test_wait_timeout": (C.c_int, [vp, C.c_uint]),
+        "hgpm_test_green": (C.c_int, [C.c_int, P(C.c_double), P(C.c_int64), P(C.c_int64)]),
         "hgpm_sizeof_params": (C.c_size_t, []),
         "hgpm_sizeof_timestepper": (C.c_size_t, []),
     }

@@ -176,4 +176,30 @@ cudaError_t launch_xpotential(int ng, const float2* in, float2* out, int zs, con
     return cudaErrorInvalidValue;
 }
 
+// Over every sum of three entries of cosq: how many of green()'s floats are not
+// the division's (out[0]), and the most float steps between the two (out[1]).
+__global__ void green_check_kernel(int ng, const double* __restrict__ cosq, double coeff,
+                                   unsigned long long* __restrict__ out) {
+    const int iz = blockIdx.x * blockDim.x + threadIdx.x, iy = blockIdx.y;
+    if (iz >= ng) return;
+    const double cyz = cosq[iy] + cosq[iz];
+    unsigned long long n = 0, most = 0;
+    for (int ix = 0; ix < ng; ++ix) {
+        const double s = cosq[ix] + cyz;
+        const int a = __float_as_int(green(s, coeff)), b = __float_as_int(s == 0.0 ? 0.f : (float)(coeff / s));
+        const unsigned long long d = a > b ? (unsigned long long)((long long)a - b) : (unsigned long long)((long long)b - a);
+        n += d != 0;
+        most = d > most ? d : most;
+    }
+    if (n) {
+        atomicAdd(&out[0], n);
+        atomicMax(&out[1], most);
+    }
+}
+
+cudaError_t launch_green_check(int ng, const double* cosq, double coeff, unsigned long long* out, cudaStream_t s) {
+    green_check_kernel<<<dim3(cdiv(ng, 128), ng), 128, 0, s>>>(ng, cosq, coeff, out);
+    return cudaGetLastError();
+}
+
 }  // namespace hgpm

@@ -83,6 +83,9 @@ cudaError_t launch_solve_small(int ng, unsigned long long* rho, float* out, doub
 // (launch_xpotential_tma: the same pass fed by TMA, x pass choice 1.)
 cudaError_t launch_xpotential(int ng, const float2* in, float2* out, int zs, const float2* tw, const double* cosq,
                               double coeff, cudaStream_t s, const Slots& sl = Slots{}, int nslots = 1);
+// The Green's function's quotient against a division, over every sum of three of
+// cosq's ng entries: out[0] floats that differ, out[1] the most steps apart.
+cudaError_t launch_green_check(int ng, const double* cosq, double coeff, unsigned long long* out, cudaStream_t s);
 // Force grid (F_x, F_y, F_z, 0) from the real potential by central
 // differences (the reference's -i sin(k) gradient, applied in real space).
 cudaError_t launch_gradient(int ng, const float* phi, float4* f, cudaStream_t s, const Slots& sl = Slots{},

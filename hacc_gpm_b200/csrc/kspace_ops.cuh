@@ -24,8 +24,10 @@ namespace hgpm {
 // start) and one correction by the remainder coeff - s q, exact in fused
 // arithmetic (Markstein 1990): 5 fused operations instead of a division's
 // subroutine with its range checks, which s (in [-6, -3e-6] or 0) and coeff
-// (0.5 / ng^3) never need.  The quotient is within an ulp of double, so the
-// float is the division's unless it lies that close to a rounding boundary.
+// (0.5 / ng^3) never need.  The start is good to 2^-22, the reciprocal to 2^-44,
+// the corrected quotient before its one rounding to 2^-88: in double, and so in
+// float, it is the division's unless the true one lies that close to a rounding
+// boundary.  (It is for every sum at 16, 200, 512 and 1024: hgpm_test_green.)
 __device__ __forceinline__ float green(double s, double coeff) {
     float r0;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"((float)s));

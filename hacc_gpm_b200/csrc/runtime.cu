@@ -534,6 +534,25 @@ extern "C" int hgpm_test_wait_timeout(hgpm_ctx* c, unsigned polls) {
     return HGPM_OK;
 }
 
+extern "C" int hgpm_test_green(int ng, const double* cosq, int64_t* n_diff, int64_t* max_steps) {
+    if (ng <= 0 || ng > 1024 || !cosq || !n_diff || !max_steps) return HGPM_ERR_ARG;
+    char* d = nullptr;
+    const size_t tab = (size_t)ng * sizeof(double);
+    if (cudaMalloc(&d, 16 + tab) != cudaSuccess) return HGPM_ERR_OOM;
+    unsigned long long out[2] = {0, 0};
+    cudaError_t e = cudaMemcpy(d, out, 16, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + 16, cosq, tab, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = launch_green_check(ng, reinterpret_cast<const double*>(d + 16), 0.5 / ((double)ng * ng * ng),
+                               reinterpret_cast<unsigned long long*>(d), nullptr);
+    if (e == cudaSuccess) e = cudaMemcpy(out, d, 16, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) return HGPM_ERR_CUDA;
+    *n_diff = (int64_t)out[0];
+    *max_steps = (int64_t)out[1];
+    return HGPM_OK;
+}
+
 // ===========================================================================
 // state I/O
 // ===========================================================================

@@ -380,6 +380,14 @@ int hgpm_tune_cache_store(const char* path, const char* device, int sms, int ng,
  * take that path without a fault.                                         */
 int hgpm_test_wait_timeout(hgpm_ctx* ctx, unsigned polls);
 
+/* ---- the Green's function's quotient, for tests -------------------------------
+ * No counterpart in the reference.  The x passes form (float)(coeff / s), coeff
+ * = 0.5 / ng^3, by an iteration of their own.  This forms it for every sum s of
+ * three entries of cosq (host, ng of them, each <= 0; ng <= 1024) both that way
+ * and by a division, on the current device, and returns how many floats differ
+ * and by how many float steps at most.                                    */
+int hgpm_test_green(int ng, const double* cosq, int64_t* n_diff, int64_t* max_steps);
+
 /* ---- ABI checks ------------------------------------------------------------
  * sizeof of the public structs, for bindings that mirror them.            */
 size_t hgpm_sizeof_params(void);

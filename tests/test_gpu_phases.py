@@ -763,3 +763,22 @@ def test_line_tiles_of_small_sides_equal_tma(ng, np_side, var, values, monkeypat
             out.append(s.store_state())
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
     assert not np.array_equal(out[0][1], v)
+
+
+@pytest.mark.parametrize("ng", [16, 24, 200, 512, 1000, 1024])
+@pytest.mark.parametrize("rounded", [True, False])
+def test_green_quotient_equals_division(ng, rounded):
+    """The Green's function's quotient is the float of the double division for
+    every mode of a side, with the cosines of rounded arguments and the exact
+    ones.  Its error before the last rounding is below 2^-88, so that none of
+    the 10^9 modes is expected to round otherwise (2^-35 of them in double, of
+    which 2^-29 in float)."""
+    if rounded:
+        cosq = np.cos((np.arange(ng, dtype=np.float32) * np.float32(2 * np.pi / ng)).astype(np.float64)) - 1.0
+    else:
+        cosq = -2.0 * np.sin(np.pi * np.arange(ng) / ng) ** 2
+    cosq = np.ascontiguousarray(cosq)
+    n, most = ctypes.c_int64(-1), ctypes.c_int64(-1)
+    rc = H.lib().hgpm_test_green(ng, cosq.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), ctypes.byref(n),
+                                 ctypes.byref(most))
+    assert rc == 0 and n.value == 0 and most.value == 0, (rc, n.value, most.value)
