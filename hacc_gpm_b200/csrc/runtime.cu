@@ -1008,12 +1008,13 @@ extern "C" int hgpm_get_force(hgpm_ctx* c, float* f) {
         // a solve may have formed none, the first halves of the paired records
         const int ng = c->ng;
         float2* phi = c->fspec + (size_t)ng * ng * c->zs;
-        if (solve_small_supported(ng))
+        if (solve_small_supported(ng)) {
             CK(cudaMemcpy2DAsync(phi, 8, c->force, 16, 8, c->ncell / 2, cudaMemcpyDeviceToDevice, c->stream));
-        else
+        } else {
             CK(launch_zinv(ng, c->fspec, reinterpret_cast<float*>(phi), ng * ng, c->zs, 0, 0, 1, 1.0f, c->tw_ng,
                            c->stream));
-        count(c, PH_ZINV, 1);
+            count(c, PH_ZINV, 1);
+        }
         c->phi_valid = true;
     }
     if (!c->force_valid && c->phi_valid) {

@@ -782,3 +782,17 @@ def test_green_quotient_equals_division(ng, rounded):
     rc = H.lib().hgpm_test_green(ng, cosq.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), ctypes.byref(n),
                                  ctypes.byref(most))
     assert rc == 0 and n.value == 0 and most.value == 0, (rc, n.value, most.value)
+
+
+@pytest.mark.parametrize("ng,kernels", [(32, 1), (64, 2)])
+def test_force_grid_on_demand_counts_its_kernels(ng, kernels):
+    """hgpm_kernel_launches counts kernels: the force grid formed after a solve is
+    the gradient alone where the potential is copied out of the paired records,
+    the z pass and the gradient elsewhere."""
+    with make(ng) as s:
+        s.load_state(*lattice_state(ng, ng))
+        s.cic()
+        s.solve_gradient()
+        s.kernel_launches(reset=True)
+        s.get_force()
+        assert s.kernel_launches() == kernels
