@@ -152,6 +152,8 @@ def kernel_names(tuned, np_side, ng, plane=None):
         "fft_z_inv": zinv,
         "kick_drift": KICK_NAMES[blk][kick],
     }
+    if blk == 16 and np_side <= 96 and kick in (5, 6, 7):
+        names["kick_drift"] = "kick_phi_kernel<16,128,1,%d> (128 particles per CTA)" % (kick == 7)
     if plane and ng in (256, 512, 1024):
         # HGPM_PLANE=1: the z and y passes in one kernel, a cluster per x plane
         names["fft_z_fwd"] = "zy_fwd_kernel<NG,3> (z and y passes, an 8-CTA cluster per x plane)"

@@ -1,9 +1,9 @@
 // ===========================================================================
 // Multi-class FFT passes (multi_class.h): one launch per pass over the work
-// units of every class and slot, one CTA per unit.  The body is the one the
-// single-class kernel runs (the z passes with 256 threads, the y and x passes
-// with 512, for every size: a butterfly's arithmetic does not depend on which
-// thread does it).
+// units of every class and slot, one CTA of 256 threads per unit.  The inverse
+// z pass runs the single-class kernel's body; the forward z pass and the flat y
+// and x tiles are this file's own.  The bits are the single-class passes' all
+// the same: a butterfly's arithmetic does not depend on which thread does it.
 // ===========================================================================
 #include <cuda_runtime.h>
 #include <stdint.h>

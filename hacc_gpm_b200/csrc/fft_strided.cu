@@ -22,10 +22,11 @@ using YT = LineTile<NG, NG <= 64 ? 1024 : NG <= 128 ? 2048 : NG <= 256 ? 4096 : 
 // 640: 616 / 617, 539 / 537; 768: 973 / 979, 1047 / 1013; 800: 1773 / 1762,
 // 1549 / 1525; 960: 2309 / 1957, 2384 / 2363; 1000: 6951 / 6927, 2609 / 2625;
 // 1024: 2242 / 2247, 2182 / 2132; 128: 12 / 12, 15 / 15; below alike, and line
-// tiles need no tensor map.  The TMA-fed pass overlaps a tile's transform with
-// the next one's load; where a plan has two radix-5 stages, or the tile of a
-// long line is 4 columns wide (32 bytes a row), the line tiles' fewer
-// exchanges and wider rows win.
+// tiles need no tensor map.  The list is these measurements, not a rule in the
+// side: the TMA-fed pass overlaps a tile's transform with the next one's load,
+// the line tiles exchange less and, at long lines, have rows twice as wide.
+// They win by most with two or three radix-5 stages (200, 400, 800, 1000), by
+// a tenth at 120, 160, 240 and 640; at 320, 768, 960 and 1024 the two are close.
 bool ypass_tma_default(int ng) {
     switch (ng) {
         case 128: case 192: case 256: case 320: case 384: case 480: case 512: case 768: case 960:

@@ -1,6 +1,7 @@
-// kspace_ops.cuh — k-space operators applied by the fused x passes:
-// pre() once per mode on the forward-transformed x line, comp(d) per output
-// component before the inverse x transform.
+// kspace_ops.cuh — k-space operators applied by the fused x passes: the
+// potential's apply() once per mode between the two x transforms; the initial
+// conditions' pre() likewise, and comp(d) per output component before the
+// inverse one.
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
@@ -40,9 +41,6 @@ __device__ __forceinline__ float green(double s, double coeff) {
 struct PotentialOp {
     const double* cosq;  // cos(k_i) - 1, one entry per grid index
     double coeff;        // 0.5 / ng^3
-    __device__ __forceinline__ float2 pre(int ix, int iy, int iz, float2 v) const {
-        return apply(__ldg(&cosq[ix]), __ldg(&cosq[iy]) + __ldg(&cosq[iz]), v);
-    }
     // cx: the x term, cyz: the sum of the y and z terms
     __device__ __forceinline__ float2 apply(double cx, double cyz, float2 v) const {
         const float g = green(cx + cyz, coeff);

@@ -1888,7 +1888,12 @@ static int deposit_candidates(int cap_default, bool w32, DepositCfg* out) {
 // windows (6.9 ms for 512^3 particles on a 1024^3 grid, against 8.3-11.8 for
 // the other windows), otherwise the column kernel (returned-value wraps 103.6
 // us at 200^3, window-sum check 106.7).  A batched launch has the blocks of
-// all its slots.
+// all its slots.  The bounds hold at the end of a run too, with cells of 1000
+// particles (100 steps to z = 0, 2 Mpc/h cells; the column kernel as it is
+// here, without a spill pass): 16^3 blocks 24 / 9 at 32^3, 31 / 27 at 64^3, 52 /
+// 51 at 96^3, 96 / 101 at 128^3; 8^3 blocks 15 / 7 at 24^3, 18 / 13 at 40^3, 46 /
+// 95 at 120^3; twice the side of cells 27 / 10 for 32^3, 50 / 21 for 64^3, 226 /
+// 130 for 128^3.
 //   Blocks left over by the column kernels (too wide, or wrapped): the spill
 // pass and its counters cost every step three launches (8 us); adding the
 // particles straight to the grid costs the deposit itself most where there are
@@ -1896,7 +1901,8 @@ static int deposit_candidates(int cap_default, bool w32, DepositCfg* out) {
 // 27 / 35 at 120^3, 95 / 103 at 200^3 (a clustered step, 100 steps on: 132 /
 // 161 and 462 / 580); 16^3 blocks 33 / 40 at 128^3, 150 / 152 at 256^3 (a
 // clustered step 948 / 916), 1085 / 1062 at 512^3.  So 8^3 blocks add
-// straight, and 16^3 blocks up to 512 of them.
+// straight, and 16^3 blocks up to 512 of them (128^3 at the end of such a run:
+// 96 / 97).
 static bool deposit_straight(int choice, int np_side, int nslots) {
     return choice == 8 && (long long)(np_side / 16) * (np_side / 16) * (np_side / 16) * nslots <= 512;
 }
@@ -2242,7 +2248,8 @@ __global__ void __launch_bounds__(256, 4) mc_deposit_kernel(const __grid_constan
     if (c.np <= 32) {
         // blocks of half the box's side: their windows reach around most of
         // it and overflow into the spill pass (24 us a step for it alone), so
-        // these add straight to the grid
+        // these add straight to the grid (at the end of a run too: one such box
+        // 9 against 24 us, deposit_default_choice)
         const ParticleSoA p = offset_soa(c.p, (size_t)slot * c.part_stride + (size_t)blk * 4096);
         unsigned long long* rho = c.rho64 + (size_t)slot * c.ncell;
         for (int i = threadIdx.x; i < 4096; i += 256)

@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kTmaThreads, 2) strided_tma_kernel(const __gri
 // x pass fused with the Green's function, persistent and TMA-fed: the next
 // x-line tile (all kx of one ky, CT kz columns) streams in while the current
 // one is transformed forward, multiplied by G (calcGreens.hpp:11-25, as
-// PotentialOp::pre) and transformed back; the potential's x-inverted spectrum
+// PotentialOp) and transformed back; the potential's x-inverted spectrum
 // leaves with coalesced streaming stores.
 template <int NG, int CT, int NT>
 __device__ __forceinline__ void store_rows(const float2* __restrict__ tile, float2* __restrict__ g, size_t rs,
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) xpotential_tma_kernel(const __gr
         const TileIdx ti = tile_of(t, nchunks, NG);
         const int iy = ti.plane, col0 = ti.chunk * CT;
         float2* tile = in[cur];
-        // forward x FFT, t = G rho_k (PotentialOp::pre with the table in
+        // forward x FFT, t = G rho_k (PotentialOp with the table in
         // shared memory, in registers between the two transforms), the
         // potential's inverse x FFT; the gradient is taken in real space
         // (gradient_kernel)
