@@ -1894,6 +1894,16 @@ static int deposit_candidates(int cap_default, bool w32, DepositCfg* out) {
 // 51 at 96^3, 96 / 101 at 128^3; 8^3 blocks 15 / 7 at 24^3, 18 / 13 at 40^3, 46 /
 // 95 at 120^3; twice the side of cells 27 / 10 for 32^3, 50 / 21 for 64^3, 226 /
 // 130 for 128^3.
+//   More particles than cells meet in the same words of the grid: us early in
+// a run and at its end, column / direct, 48^3 on 24^3 13, 18 / 9, 20; 64^3 on
+// 32^3 13, 38 / 15, 42; 80^3 on 40^3 13, 19 / 20, 61; 96^3 on 48^3 17, 27 / 26, 89;
+// 8^3 blocks 40^3 on 24^3 9, 13 / 9, 17.  So these go direct up to 27 blocks.
+// A few more cells than particles a side (below half as many again) likewise,
+// once there are 1000 blocks, and there the column kernel beats the 13312-cell
+// windows too: early, late, column / windows / direct, 80^3 on 96^3 15, 27 / 24,
+// 37 / 18, 36; 96^3 on 128^3 23, 41 / 34, 53 / 27, 51; 120^3 on 128^3 28, 49 / 44,
+// 65 / 38, 93; 128^3 on 160^3 37, 68 / 58, 85 / 51, 103; on 192^3 47, 88 / 68, 119 /
+// 55, 98, on 256^3 - / 116, 226 / 113, 130.
 //   Blocks left over by the column kernels (too wide, or wrapped): the spill
 // pass and its counters cost every step three launches (8 us); adding the
 // particles straight to the grid costs the deposit itself most where there are
@@ -1910,9 +1920,9 @@ static bool deposit_straight(int choice, int np_side, int nslots) {
 template <int B>
 static int deposit_default_choice(int np_side, int ng, int nslots) {
     const long long blocks = (long long)(np_side / B) * (np_side / B) * (np_side / B) * nslots;
-    if (B == 16) return blocks <= 216 ? 9 : 8;
-    if (ng > np_side) return blocks <= 4096 ? 5 : 1;
-    return blocks <= 512 ? 5 : 4;
+    if (B == 16) return blocks <= (np_side > ng ? 27 : 216) ? 9 : 8;
+    if (ng > np_side) return blocks > 4096 ? 1 : 2 * ng < 3 * np_side && blocks > 512 ? 4 : 5;
+    return blocks <= (np_side > ng ? 27 : 512) ? 5 : 4;
 }
 
 template <int B, bool SMALL>

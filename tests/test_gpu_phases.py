@@ -796,3 +796,34 @@ def test_force_grid_on_demand_counts_its_kernels(ng, kernels):
         s.kernel_launches(reset=True)
         s.get_force()
         assert s.kernel_launches() == kernels
+
+
+@pytest.mark.parametrize("np_side,ng,choice", [
+    (48, 24, 9), (64, 32, 8), (64, 48, 8), (80, 40, 8), (96, 48, 8), (96, 96, 9), (24, 16, 5),
+    (40, 24, 4), (40, 40, 5), (64, 80, 5), (80, 96, 4), (96, 128, 4), (96, 160, 5), (120, 128, 4), (128, 160, 4),
+    (128, 192, 5), (160, 192, 1), (200, 240, 1)])
+def test_deposit_of_boxes_around_the_direct_rule(np_side, ng, choice, monkeypatch):
+    """Which deposit a box takes by its blocks and its particles a cell (adding
+    straight to the grid loses where many particles meet in a cell), and that
+    its density is the window deposit's, bit for bit, with the particles drawn
+    together too."""
+    for k in ("HGPM_DEPOSIT", "HGPM_KICK"):
+        monkeypatch.delenv(k, raising=False)
+    monkeypatch.setenv("HGPM_NO_TUNE_CACHE", "1")
+    x, v = lattice_state(np_side, ng, disp=0.7, seed=3)
+    c = np.float32(ng / 2)
+    clumped = np.mod(c + (x - c) * np.float32(0.2), np.float32(ng)).astype(np.float32)
+    clumped[clumped >= ng] = 0
+    got = []
+    for force in (None, "0"):
+        if force is not None:
+            monkeypatch.setenv("HGPM_DEPOSIT", force)
+        with make(ng, np_side) as s:
+            assert s.tuned_choices()["deposit"] == (choice if force is None else 0)
+            rho = []
+            for state in (x, clumped):
+                s.load_state(state, v)
+                s.cic()
+                rho.append(s.get_density())
+        got.append(rho)
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
