@@ -2051,7 +2051,10 @@ int kick_kernels(int choice, int np_side, int ng) {
 // overlap, kicks of 512^3 took 7-12 ms instead of 2.0.  Several waves leave
 // the balance to the block scheduler: 512^3 alone 2.00 / 2.04 / 2.05 / 2.06
 // ms a kick in 1 / 2 / 4 / 8 waves, four steps of three contexts in turn
-// 28.5 / 25.7 / 23.7 / 24.2 ms.  With more cells than particles a side
+// 28.5 / 25.7 / 23.7 / 24.2 ms.  What it costs a context that has the GPU to
+// itself is a CTA's turnover a wave, 6 to 15 us: 254 -> 274 us at 256^3, 492 ->
+// 522 at 320^3, 2030 -> 2075 at 512^3 (CTAs of 512 or 256 threads, two or four an
+// SM, hide it but lose more: 268 / 281, 578 / 530, 2326 / 2390).  With more cells than particles a side
 // (8^3 blocks, CTAs of 256 threads whose turnover hides behind the other
 // three of the SM) short shares also keep the resident CTAs' gathers close
 // together: 512^3 particles on 1024^3 4.77 / 4.19 / 3.70 / 3.34 ms in 1 / 4 /
